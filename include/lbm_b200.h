@@ -292,7 +292,9 @@ int lbm_mass_momentum_noalloc(const float* f, int32_t nx, int32_t ny, int32_t nz
  * AR(1) (correlation 0.98) and normalised to zero mean and unit standard deviation
  * from level 1 on.  The random phases come from a counter-based hash of seed (the
  * reference draws them from the compiler's random_number).  Synchronises the
- * context's stream before it returns (it frees its temporaries). */
+ * context's stream before it returns.  The context keeps the transform's plan and a
+ * buffer of at most 64 MiB (or of eight levels, where those are larger) until it is
+ * destroyed. */
 int lbm_inflow_turbulence_compute(lbm_ctx* ctx, float* uu, float* vv, float* ww, float* rr, int32_t nrturb,
                                   uint64_t seed);
 

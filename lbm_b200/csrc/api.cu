@@ -10,6 +10,8 @@
 #include <type_traits>
 #include <vector>
 
+#include <cufft.h>
+
 #include "../../include/lbm_b200.h"
 #include "boundary.cuh"
 #include "ref_kernels.cuh"
@@ -76,6 +78,10 @@ struct lbm_ctx {
     int* d_it = nullptr;          // number of the step being computed
     int* d_status = nullptr;
     float* d_adj_terms = nullptr; // 4 x cells: the macrovars adjoint terms of lbm_macrovars_drift_adj (allocated on first use)
+    float* d_turb_buf = nullptr;  // planes of the inflow-turbulence generator (allocated on first use)
+    double* d_turb_part = nullptr;   // its block sums
+    cufftHandle turb_plan = 0;    // its transform, valid while turb_planes > 0
+    int turb_planes = 0;
     double* d_partial = nullptr;  // FP64 block partials of the conservation sums (scratch)
     double* d_sum = nullptr;      // their total (4 doubles)
     int it = 0;
@@ -891,6 +897,9 @@ int lbm_destroy(lbm_ctx* c) {
     for (int b = 0; b < 2; ++b) cudaFree(c->d_xg[b]);
     cudaFree(c->d_abl);
     cudaFree(c->d_adj_terms);
+    if (c->turb_planes > 0) cufftDestroy(c->turb_plan);
+    cudaFree(c->d_turb_buf);
+    cudaFree(c->d_turb_part);
     cudaFree(c->d_it);
     cudaFree(c->d_status);
     cudaFree(c->d_partial);

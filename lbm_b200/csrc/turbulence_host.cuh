@@ -1,9 +1,45 @@
 // turbulence_host.cuh -- C ABI of the GPU inflow-turbulence generator
 // (declaration in include/lbm_b200.h).  Included at the end of api.cu.
 
-#include <cufft.h>
-
 #include "turbulence.cuh"
+
+namespace {
+
+// Bytes of the transform buffer a context keeps, unless one group of levels needs
+// more: the levels go through it in chunks, so its size does not grow with nrturb,
+// and a chunk stays in L2 between the spectrum, the transform and the chain.
+constexpr size_t kTurbBufBytes = 64u << 20;
+
+void turb_release(lbm_ctx* c) {
+    if (c->turb_planes > 0) cufftDestroy(c->turb_plan);
+    cudaFree(c->d_turb_buf);
+    cudaFree(c->d_turb_part);
+    c->turb_planes = 0;
+    c->d_turb_buf = nullptr;
+    c->d_turb_part = nullptr;
+}
+
+// the transform's plan and buffer for `planes` planes of the context's size, kept
+// until the context is destroyed or a call needs another number of planes (making
+// them on each call cost 3 to 14 ms)
+int turb_workspace(lbm_ctx* c, int planes, int n1, int n2) {
+    if (c->turb_planes == planes) return LBM_OK;
+    turb_release(c);
+    int rc = cuda_check(c, cudaMalloc(&c->d_turb_buf, (size_t)planes * n2 * (n1 / 2 + 1) * sizeof(float2)),
+                        "cudaMalloc(turbulence planes)");
+    if (rc == LBM_OK)
+        rc = cuda_check(c, cudaMalloc(&c->d_turb_part, (size_t)8 * LBM_TURB_MAXBLK * LBM_TURB_NS * sizeof(double)),
+                        "cudaMalloc(turbulence sums)");
+    int n[2] = {n2, n1};
+    if (rc == LBM_OK &&
+        cufftPlanMany(&c->turb_plan, 2, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, planes) != CUFFT_SUCCESS)
+        rc = fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftPlanMany failed");
+    if (rc == LBM_OK) c->turb_planes = planes;
+    else turb_release(c);
+    return rc;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -23,65 +59,70 @@ int lbm_inflow_turbulence_compute(lbm_ctx* c, float* uu, float* vv, float* ww, f
     const double deltak = pi2 * pi2 / ((double)n1 * n2);
     const double kappa2 = (pi2 / n1) * (pi2 / n1), lambda2 = (pi2 / n2) * (pi2 / n2);
     const double r1 = sqrt(8.0) / rx, r2 = sqrt(8.0) / rx;   // the reference derives both from rx
-    double summ = 0.0;
-    for (int p = -n2 / 2 + 1; p <= n2 / 2; ++p)
-        for (int l = -n1 / 2 + 1; l <= n1 / 2; ++l)
-            summ += exp(-2.0 * (kappa2 * l * l / (r1 * r1) + lambda2 * p * p / (r2 * r2)));
+    // the sum over the wavenumbers is a product of two one-dimensional sums
+    double sum1 = 0.0, sum2 = 0.0;
+    for (int l = -n1 / 2 + 1; l <= n1 / 2; ++l) sum1 += exp(-2.0 * (kappa2 * l * l / (r1 * r1)));
+    for (int p = -n2 / 2 + 1; p <= n2 / 2; ++p) sum2 += exp(-2.0 * (lambda2 * p * p / (r2 * r2)));
+    double summ = sum1 * sum2;
     summ -= 1.0;   // the mean is not sampled
     const double cc = sqrt(1.0 / (deltak * summ));
     TurbSpec s;
     s.n1 = n1;
     s.n2 = n2;
-    s.nb = nf * (nrturb + 1);
+    s.nt = nrturb + 1;
     s.amp = (float)(sqrt(deltak) * cc);
     s.ak = (float)(kappa2 / (r1 * r1));
     s.al = (float)(lambda2 / (r2 * r2));
     s.seed = seed;
 
+    // chunks of whole groups of levels, of about equal length
+    const int groups = nrturb / LBM_TURB_B + 1;
+    const size_t group_bytes = (size_t)nf * LBM_TURB_B * n2 * (n1 / 2 + 1) * sizeof(float2);
+    const int per = (int)std::max<size_t>(1, std::min<size_t>(groups, kTurbBufBytes / group_bytes));
+    const int nchunk = (groups + per - 1) / per;
+    const int gchunk = (groups + nchunk - 1) / nchunk;
+    const int C = gchunk * LBM_TURB_B, planes = nf * C;
+    LBM_TRY(turb_workspace(c, planes, n1, n2));
+    if (cufftSetStream(c->turb_plan, c->stream) != CUFFT_SUCCESS)
+        return fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftSetStream failed");
+    TurbChain ch;
+    ch.Y = c->d_turb_buf;
+    float* outs[4] = {uu, vv, ww, rr};
+    for (int f = 0; f < 4; ++f) ch.o[f] = outs[f];
+    ch.part = c->d_turb_part;
+    ch.ny = ny;
+    ch.nz = nz;
+    ch.n2 = n2;
+    ch.pitch = 2 * (n1 / 2 + 1);   // an in-place transform leaves its rows at the spectrum's pitch
+    ch.C = C;
+    ch.nrturb = nrturb;
+    // the plane is small (two state buffers of 36 or more elements per row and direction fit the
+    // card), so 32-bit indices hold it; about four cells per thread
+    const int nblk = std::min(LBM_TURB_MAXBLK, (ny * nz + 4 * LBM_TURB_T - 1) / (4 * LBM_TURB_T));
+    const int h = n1 / 2 + 1;
+    const dim3 sgrd((unsigned)((n2 * h + 255) / 256), (unsigned)((planes + LBM_TURB_LPT - 1) / LBM_TURB_LPT));
     int rc = LBM_OK;
-    float2* X = nullptr;
-    float* Y = nullptr;
-    float** outs = nullptr;
-    cufftHandle plan = 0;
-    bool planned = false;
-    const size_t nx_c = (size_t)s.nb * n2 * (n1 / 2 + 1), ny_r = (size_t)s.nb * n2 * n1;
-    auto chk = [&](cudaError_t e, const char* w) {
-        if (rc == LBM_OK && e != cudaSuccess) rc = cuda_check(c, e, w);
-    };
-    chk(cudaMalloc(&X, nx_c * sizeof(float2)), "cudaMalloc(turbulence spectrum)");
-    chk(cudaMalloc(&Y, ny_r * sizeof(float)), "cudaMalloc(turbulence fields)");
-    chk(cudaMalloc(&outs, 4 * sizeof(float*)), "cudaMalloc(turbulence outputs)");
-    if (rc == LBM_OK) {
-        float* h[4] = {uu, vv, ww, rr};
-        chk(cudaMemcpyAsync(outs, h, 4 * sizeof(float*), cudaMemcpyHostToDevice, c->stream), "turbulence outputs");
-    }
-    if (rc == LBM_OK) {
-        int n[2] = {n2, n1};
-        if (cufftPlanMany(&plan, 2, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, s.nb) != CUFFT_SUCCESS)
-            rc = fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftPlanMany failed");
-        else planned = true;
-        if (rc == LBM_OK && cufftSetStream(plan, c->stream) != CUFFT_SUCCESS)
-            rc = fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftSetStream failed");
-    }
-    if (rc == LBM_OK) {
-        k_turb_spectrum<<<(unsigned)((nx_c + 255) / 256), 256, 0, c->stream>>>(X, s);
+    for (int g0 = 0; g0 < groups && rc == LBM_OK; g0 += gchunk) {
+        const int g1 = std::min(groups, g0 + gchunk);
+        ch.t0 = g0 * LBM_TURB_B;
+        k_turb_spectrum<<<sgrd, 256, 0, c->stream>>>((float2*)c->d_turb_buf, s, ch.t0, C, planes);
         c->launches++;
-        chk(cudaGetLastError(), "turbulence spectrum");
+        rc = cuda_check(c, cudaGetLastError(), "turbulence spectrum");
+        if (rc == LBM_OK &&
+            cufftExecC2R(c->turb_plan, reinterpret_cast<cufftComplex*>(c->d_turb_buf), c->d_turb_buf) != CUFFT_SUCCESS)
+            rc = fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftExecC2R failed");
+        // sums of the chunk's first group; then each group's levels with the next group's
+        // sums; the last group's levels while its planes are still in the buffer
+        for (int g = g0 - 1; g < g1 && rc == LBM_OK; ++g) {
+            const int ga = g < g0 ? -1 : g, gc = g + 1 < g1 ? g + 1 : -1;
+            rc = cuda_check(c, launch_pdl(k_turb_chain, dim3(nblk, nf), dim3(LBM_TURB_T), c->stream, ch, ga, gc),
+                            "turbulence levels");
+            c->launches++;
+        }
     }
-    if (rc == LBM_OK && cufftExecC2R(plan, reinterpret_cast<cufftComplex*>(X), Y) != CUFFT_SUCCESS)
-        rc = fail(c, LBM_ERR_CUDA, "inflow_turbulence_compute: cufftExecC2R failed");
-    if (rc == LBM_OK) {
-        k_turb_ar1<1024><<<nf, 1024, 0, c->stream>>>(Y, outs, ny, nz, n1, n2, nrturb);
-        c->launches++;
-        chk(cudaGetLastError(), "turbulence levels");
-    }
-    // the temporaries are released after the work that uses them
-    if (X || Y || outs) chk(cudaStreamSynchronize(c->stream), "inflow_turbulence_compute");
-    if (planned) cufftDestroy(plan);
-    cudaFree(X);
-    cudaFree(Y);
-    cudaFree(outs);
-    return rc;
+    // the caller may read the fields from any stream once this returns
+    const int rs = cuda_check(c, cudaStreamSynchronize(c->stream), "inflow_turbulence_compute");
+    return rc != LBM_OK ? rc : rs;
 }
 
 }  // extern "C"
