@@ -696,11 +696,20 @@ int postcoll_run(lbm_ctx* c, R* f, R* tau, const R* rho, const R* u, const R* v,
     return LBM_OK;
 }
 
+template <int Q, typename R>
+int drift_launch(lbm_ctx* c, R* f, const R* feq) {
+    using D = DriftTile<Q, R>;
+    const DriftShape d = drift_shape<Q, R>(c->rg, c->nsm * D::BLOCKS);
+    const dim3 grd((c->p.nx + d.ni - 1) / d.ni * ((c->p.ny + D::TJ - 1) / D::TJ), (c->p.nz + d.ks - 1) / d.ks);
+    LBM_TRY(cuda_check(c, cudaFuncSetAttribute(k_ref_drift<Q, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D::SMEM),
+                       "drift"));
+    k_ref_drift<Q, R><<<grd, D::T, D::SMEM, c->stream>>>(f, feq, c->rg, d);
+    return LBM_OK;
+}
 template <typename R>
 int drift_run(lbm_ctx* c, R* f, const R* feq) {
     if (f == feq) return fail(c, LBM_ERR_ARG, "drift: f and feq must be distinct buffers");
-    if (c->p.nl == 27) k_ref_drift<27, R><<<dim3(c->p.ny, c->p.nz), 256, 0, c->stream>>>(f, feq, c->rg);
-    else k_ref_drift<19, R><<<dim3(c->p.ny, c->p.nz), 256, 0, c->stream>>>(f, feq, c->rg);
+    LBM_TRY(c->p.nl == 27 ? drift_launch<27, R>(c, f, feq) : drift_launch<19, R>(c, f, feq));
     c->launches++;
     LBM_LAUNCHED(c, "drift");
     return LBM_OK;

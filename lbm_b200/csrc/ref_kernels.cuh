@@ -13,6 +13,7 @@
 #pragma once
 
 #include "collide.cuh"
+#include "ref_tiles.cuh"
 
 namespace lbm {
 
@@ -149,38 +150,140 @@ __global__ void __launch_bounds__(128) k_ref_postcoll(R* f, R* tau, const R* rho
     tile_store<Q>(sm, f, g.cell(i0, j, k), n);
 }
 
-// drift: f(l,i,j,k) = feq(l,i-cx,j-cy,k-cz) over interior cells; a thread per
-// (l,i) of a row, as m_drift_kernel.F90:33-42 flattens it.  The source of
-// element e = (i-1) Q + l of a row is e minus the direction's distance Q d_l,
-// d_l = cx + (nx+2) cy + (nx+2)(ny+2) cz, taken from shared memory (a constant
-// read would serialise over the different l of a warp).  Each thread keeps
-// DRIFT_ILP loads in flight before its stores.
-#define DRIFT_ILP 4
-template <int Q, typename R = float>
-__global__ void __launch_bounds__(256) k_ref_drift(R* __restrict__ f, const R* __restrict__ feq, RefGrid g) {
-    // one block per interior row (j,k), looping over its nx*Q outputs
-    __shared__ long long sd[Q];
-    if (threadIdx.x < Q) {
-        const int l = threadIdx.x;
-        sd[l] = (long long)Q * (lat_cx(l) + (long long)lat_cy(l) * (g.nx + 2) +
-                                (long long)lat_cz(l) * (g.nx + 2) * (g.ny + 2));
+// drift: f(l,i,j,k) = feq(l,i-cx,j-cy,k-cz) over interior cells
+// (m_drift_kernel.F90:33-42).
+//
+// A direction's values lie nl elements apart, so gathering them from global
+// memory takes one 32-byte sector per element (347 us for D3Q27 256x128x128
+// FP32, 2.6 TB/s of the bytes it must move; 140 us for D3Q19 192x96x96 FP64).
+// Instead a block owns TJ rows of NI cells and marches along k with a ring of
+// planes of its rows and their neighbours in shared memory: the three that an
+// output plane needs and the next ones, still arriving.  A source row crosses L2
+// about 1.6 times ((TJ+2)/TJ (NI+2)/NI) instead of nine, all copies are whole
+// 16-byte words, and a thread writes one direction: its source sits at a fixed
+// distance.
+//
+// A row of the ring starts at the phase its global address has in a word
+// (ref_tiles.cuh): the row stride rs equals the global one modulo a word, and a
+// plane is placed at its own phase.  The words at a row's ends bring up to a
+// word of its neighbours along; only at the two ends of the array, where a word
+// could reach past it, do they move element by element.
+template <int Q, typename R>
+struct DriftTile {
+    static constexpr int TJ = (sizeof(R) == 8 && Q == 27) ? 3 : 4;
+    static constexpr int NI = 128 / (int)sizeof(R);            // cells of a row: 32 FP32, 16 FP64
+    static constexpr int SLOTS = Q == 27 ? 5 : 6;              // planes of the ring: two blocks fill an SM
+    static constexpr int AHEAD = SLOTS - 3;                    // planes under way
+    static constexpr int LANES = 16;                           // cells per pass of a block
+    static constexpr int T = Q * LANES;                        // a thread per (cell, direction)
+    static constexpr int V = word_elems<R>();
+    static constexpr int ROW = (NI + 2) * Q;                   // elements of a row, at most
+    static constexpr int WORDS = (ROW + 2 * (V - 1)) / V;      // words a row may touch
+    static constexpr int RS = (WORDS + 2) * V;                 // row stride, at most
+    static constexpr int PS = (TJ + 2) * RS + V;               // plane stride
+    static constexpr size_t SMEM = (size_t)SLOTS * PS * sizeof(R);
+    static constexpr int BLOCKS = 2;
+    static_assert(BLOCKS * (SMEM + 1024) <= 228 * 1024, "the blocks fit an SM");
+};
+struct DriftShape {
+    int ni;        // cells of a row chunk
+    int ks;        // planes of a k segment
+    int rs;        // row stride of the ring: room for a row, congruent to the global stride
+};
+template <int Q, typename R>
+DriftShape drift_shape(const RefGrid& g, int slots) {
+    using D = DriftTile<Q, R>;
+    DriftShape d;
+    const int nch = (g.nx + D::NI - 1) / D::NI;
+    d.ni = (g.nx + nch - 1) / nch;
+    const int least = (D::WORDS + 1) * D::V;
+    d.rs = least + (int)(((long long)(g.nx + 2) * Q) % D::V);
+    // segments of k: a block takes about ks + 4 plane times (two extra planes and the
+    // first ones' latency); `slots` blocks run at a time
+    const long long columns = (long long)nch * ((g.ny + D::TJ - 1) / D::TJ);
+    long long best = -1;
+    d.ks = g.nz;
+    for (int ns = 1; ns <= g.nz && ns <= 64; ++ns) {
+        const int ks = (g.nz + ns - 1) / ns;
+        const long long cost = (columns * ((g.nz + ks - 1) / ks) + slots - 1) / slots * (ks + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            d.ks = ks;
+        }
     }
-    __syncthreads();
-    const int j = blockIdx.x + 1, k = blockIdx.y + 1;
-    const long long base = g.cell(1, j, k) * Q;
-    const int n = Q * g.nx;
-    for (int e0 = threadIdx.x; e0 < n; e0 += blockDim.x * DRIFT_ILP) {
-        R v[DRIFT_ILP];
+    return d;
+}
+
+template <int Q, typename R = float>
+__global__ void __launch_bounds__(DriftTile<Q, R>::T, DriftTile<Q, R>::BLOCKS)
+    k_ref_drift(R* __restrict__ f, const R* __restrict__ feq, RefGrid g, DriftShape d) {
+    using D = DriftTile<Q, R>;
+    constexpr int V = D::V, TJ = D::TJ;
+    constexpr int LOADS = ((TJ + 2) * D::WORDS + D::T - 1) / D::T;   // words a thread copies per plane
+    extern __shared__ __align__(16) unsigned char raw[];
+    R* sm = reinterpret_cast<R*>(raw);
+    const int tid = threadIdx.x;
+    // grid: x over the chunks of a row, then the row tiles; y over the k segments
+    const int nch = (g.nx + d.ni - 1) / d.ni, jt = blockIdx.x / nch;
+    const int i0 = (blockIdx.x - jt * nch) * d.ni + 1, j0 = jt * TJ + 1, k0 = blockIdx.y * d.ks + 1;
+    const int ni = min(d.ni, g.nx + 1 - i0), nj = min(TJ, g.ny + 1 - j0), k1 = min(k0 + d.ks, g.nz + 1);
+    if (ni <= 0 || nj <= 0 || k0 >= k1) return;
+    const int np = k1 - k0;
+    const long long rowg = (long long)(g.nx + 2) * Q, planeg = rowg * (g.ny + 2);
+    const R* src = feq + g.cell(i0 - 1, j0 - 1, k0 - 1) * Q;    // first element of plane 0
+    const int len = (ni + 2) * Q, ph0 = phase_of(src);
+    // a block whose first or last row is the array's
+    const bool ends = (i0 == 1 && j0 == 1 && k0 == 1) || (i0 + ni > g.nx && j0 + nj > g.ny && k1 > g.nz);
+    // the words this thread copies of each plane: row and word within the row
+    int lr[LOADS], lw[LOADS];
 #pragma unroll
-        for (int u = 0; u < DRIFT_ILP; ++u) {
-            const int e = e0 + u * blockDim.x;
-            if (e < n) v[u] = feq[base + e - sd[e % Q]];
-        }
+    for (int q = 0; q < LOADS; ++q) {
+        const int e = tid + q * D::T;
+        lr[q] = e / D::WORDS;
+        lw[q] = e - lr[q] * D::WORDS;
+    }
+    // plane p (k = k0 - 1 + p) into ring slot `slot`
+    auto load_plane = [&](int p, int slot) {
+        const R* s = src + p * planeg;
+        const int at = slot * D::PS + phase_of(s);
 #pragma unroll
-        for (int u = 0; u < DRIFT_ILP; ++u) {
-            const int e = e0 + u * blockDim.x;
-            if (e < n) f[base + e] = v[u];
+        for (int q = 0; q < LOADS; ++q) {
+            if (lr[q] >= nj + 2) break;
+            const R* row = s + lr[q] * rowg;
+            const int o = at + lr[q] * d.rs, ph = o % V;        // element 0 of the row, and its phase
+            if (ends) run_load_word(sm + (o - ph), row, ph, len, lw[q]);
+            else if (lw[q] * V < ph + len) cp_async16(sm + (o - ph) + lw[q] * V, row - ph + lw[q] * V);
         }
+    };
+#pragma unroll
+    for (int p = 0; p < 2 + D::AHEAD; ++p) {
+        if (p < np + 2) load_plane(p, p);
+        cp_async_commit();
+    }
+    const int l = tid % Q;
+    const int cz = c_cz[l];
+    const int from = (1 - c_cy[l]) * d.rs + (1 - c_cx[l]) * Q + tid;
+    R* dst = f + g.cell(i0, j0, k0) * Q + tid;
+    const int n = ni * Q;
+    int slot = 1, next = 2 + D::AHEAD;                          // slots of the planes p + 1 and p + 2 + AHEAD
+    for (int p = 0; p < np; ++p) {                              // output plane k0 + p = plane p + 1
+        cp_async_wait<D::AHEAD - 1>();
+        __syncthreads();                                        // planes p .. p+2 are here; all are past plane p-1
+        if (p + 2 + D::AHEAD < np + 2) load_plane(p + 2 + D::AHEAD, next);
+        cp_async_commit();
+        int at = slot - cz;
+        at += at < 0 ? D::SLOTS : (at >= D::SLOTS ? -D::SLOTS : 0);
+        const R* s = sm + at * D::PS + (int)((ph0 + (p + 1 - cz) * planeg) & (V - 1)) + from;
+#pragma unroll
+        for (int r = 0; r < TJ; ++r) {
+            if (r >= nj) break;
+#pragma unroll
+            for (int m = 0; m < D::NI / D::LANES; ++m)
+                if (tid + m * D::T < n) dst[r * rowg + m * D::T] = s[r * d.rs + m * D::T];
+        }
+        dst += planeg;
+        slot = slot + 1 == D::SLOTS ? 0 : slot + 1;
+        next = next + 1 == D::SLOTS ? 0 : next + 1;
     }
 }
 
