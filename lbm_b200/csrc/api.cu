@@ -686,14 +686,29 @@ int fequil3_run(lbm_ctx* c, R* feq, const R* rho, const R* u, const R* v, const 
     return LBM_OK;
 }
 
+// a tiled kernel: `blocks` resident per SM walk the tiles
+template <typename... KArgs, typename... Args>
+int tiled_launch(lbm_ctx* c, const char* what, void (*kern)(KArgs...), size_t smem, int blocks, unsigned ntiles,
+                 Args... args) {
+    LBM_TRY(cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), what));
+    const unsigned grid = std::min(ntiles, (unsigned)(c->nsm * blocks));
+    kern<<<grid, CELL_T, smem, c->stream>>>(args..., ntiles);
+    c->launches++;
+    LBM_LAUNCHED(c, what);
+    return LBM_OK;
+}
+
+template <int Q, typename R>
+int postcoll_launch(lbm_ctx* c, R* f, R* tau, const R* rho, const R* u, const R* v, const R* w, const R* abl) {
+    using P = PostcollTile<Q, R>;
+    const unsigned tp = plane_tiles(c->rg);
+    return tiled_launch(c, "postcoll", k_ref_postcoll<Q, R>, P::SMEM, P::BLOCKS, tp * (unsigned)c->p.nz, f, tau, rho, u, v,
+                        w, abl, c->rg, cp_of<R>(c), tp);
+}
 template <typename R>
 int postcoll_run(lbm_ctx* c, R* f, R* tau, const R* rho, const R* u, const R* v, const R* w, const R* ablvisc) {
-    const CollideParamsT<R>& cp = cp_of<R>(c);
-    if (c->p.nl == 27) k_ref_postcoll<27, R><<<interior_rows(c), 128, 0, c->stream>>>(f, tau, rho, u, v, w, ablvisc, c->rg, cp);
-    else k_ref_postcoll<19, R><<<interior_rows(c), 128, 0, c->stream>>>(f, tau, rho, u, v, w, ablvisc, c->rg, cp);
-    c->launches++;
-    LBM_LAUNCHED(c, "postcoll");
-    return LBM_OK;
+    return c->p.nl == 27 ? postcoll_launch<27, R>(c, f, tau, rho, u, v, w, ablvisc)
+                         : postcoll_launch<19, R>(c, f, tau, rho, u, v, w, ablvisc);
 }
 
 template <int Q, typename R>
@@ -715,14 +730,15 @@ int drift_run(lbm_ctx* c, R* f, const R* feq) {
     return LBM_OK;
 }
 
+template <int Q, typename R>
+int macrovars_launch(lbm_ctx* c, R* rho, R* u, R* v, R* w, const R* f) {
+    using P = MacroTile<Q, R>;
+    return tiled_launch(c, "macrovars", k_ref_macrovars<Q, R>, P::SMEM, P::BLOCKS, all_tiles(c->rg), rho, u, v, w, f,
+                        c->rg);
+}
 template <typename R>
 int macrovars_run(lbm_ctx* c, R* rho, R* u, R* v, R* w, const R* f) {
-    dim3 grd((c->p.nx + 2 + 127) / 128, c->p.ny + 2, c->p.nz + 2);
-    if (c->p.nl == 27) k_ref_macrovars<27, R><<<grd, 128, 0, c->stream>>>(rho, u, v, w, f, c->rg);
-    else k_ref_macrovars<19, R><<<grd, 128, 0, c->stream>>>(rho, u, v, w, f, c->rg);
-    c->launches++;
-    LBM_LAUNCHED(c, "macrovars");
-    return LBM_OK;
+    return c->p.nl == 27 ? macrovars_launch<27, R>(c, rho, u, v, w, f) : macrovars_launch<19, R>(c, rho, u, v, w, f);
 }
 
 template <typename R>

@@ -118,36 +118,81 @@ __global__ void __launch_bounds__(128) k_ref_fequil3(R* feq, const R* rho, const
     tile_store<Q>(sm, feq, g.cell(i0, j, k), n);
 }
 
+// Shared memory and resident blocks of the tiled kernels: two tile buffers with
+// `scalars` values per cell each; as many blocks as fit an SM, up to a cap on
+// their registers.
+template <int Q, typename R>
+struct PostcollTile {
+    static constexpr int SC = 5;                                   // rho, u, v, w, tau
+    static constexpr int STAGE = CellTile<Q, R>::BUF + SC * CELL_T;    // elements of one of the two stages
+    static constexpr size_t SMEM = 2 * STAGE * sizeof(R);
+    static constexpr int BLOCKS = sizeof(R) == 4 ? (Q == 27 ? 6 : 7) : (Q == 27 ? 3 : 4);
+};
+template <int Q, typename R>
+struct MacroTile {
+    static constexpr int STAGE = CellTile<Q, R>::BUF;
+    static constexpr size_t SMEM = 2 * STAGE * sizeof(R);
+    static constexpr int BLOCKS = sizeof(R) == 4 ? (Q == 27 ? 7 : 10) : (Q == 27 ? 4 : 5);
+};
+
 // postcoll: collide interior cells in place with the given moments (m_postcoll_kernel.F90:7-255)
 template <int Q, typename R = float>
-__global__ void __launch_bounds__(128) k_ref_postcoll(R* f, R* tau, const R* rho, const R* u,
-                                                      const R* v, const R* w, const R* abl, RefGrid g,
-                                                      CollideParamsT<R> cp) {
-    __shared__ R sm[128 * Q];
-    const int i0 = blockIdx.x * 128 + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
-    const int n = min(128, g.nx + 1 - i0);
-    const int t = threadIdx.x;
-    if (n <= 0) return;
-    tile_load<Q>(sm, f, g.cell(i0, j, k), n);
-    __syncthreads();
-    if (t < n) {
-        const long long c = g.cell(i0 + t, j, k);
-        R fp[Q];
+__global__ void __launch_bounds__(CELL_T, PostcollTile<Q, R>::BLOCKS)
+    k_ref_postcoll(R* f, R* tau, const R* rho, const R* u, const R* v, const R* w, const R* abl, RefGrid g,
+                   CollideParamsT<R> cp, unsigned tp, unsigned ntiles) {
+    using P = PostcollTile<Q, R>;
+    extern __shared__ __align__(16) unsigned char raw[];
+    __shared__ unsigned cells[CELL_T / 32];
+    R* sm = reinterpret_cast<R*>(raw);
+    const int tid = threadIdx.x;
+    auto fetch = [&](unsigned t, int b) {
+        const TileAt a = tile_at<false>(g, t, tp);
+        tile_fetch<Q>(sm + b * P::STAGE, f, a.c0, a.n);
+        if (tid < a.n) {
+            R* s = sm + b * P::STAGE + CellTile<Q, R>::BUF + tid;
+            const long long c = a.c0 + tid;
+            cp_async_elem(s, rho + c);
+            cp_async_elem(s + CELL_T, u + c);
+            cp_async_elem(s + 2 * CELL_T, v + c);
+            cp_async_elem(s + 3 * CELL_T, w + c);
+            cp_async_elem(s + 4 * CELL_T, tau + c);
+        }
+    };
+    fetch(blockIdx.x, 0);
+    cp_async_commit();
+    int b = 0;
+    for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
+        if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
+        cp_async_commit();
+        const TileAt a = tile_at<false>(g, t, tp);
+        const unsigned i = (a.q0 + tid) % (unsigned)(g.nx + 2);
+        const bool inner = tid < a.n && i >= 1 && i <= (unsigned)g.nx;
+        const unsigned mask = __ballot_sync(0xffffffffu, inner);
+        if ((tid & 31) == 0) cells[tid >> 5] = mask;
+        cp_async_wait<1>();
+        __syncthreads();
+        R* tile = sm + b * P::STAGE;
+        if (inner) {
+            R* s = tile + phase_of(f + a.c0 * Q) + tid * Q;
+            const R* sc = tile + CellTile<Q, R>::BUF + tid;
+            R fp[Q];
 #pragma unroll
-        for (int l = 0; l < Q; ++l) fp[l] = sm[t * Q + l] - lat_w<Q, R>(l);
-        const MomentsT<R> m = moments<Q>(fp);
-        const R r = rho[c];
-        TurbInT<R> tb;
-        tb.on = false;
-        tb.dux = tb.duy = tb.duz = R(0);
-        const R tnew = collide<Q>(fp, m, r - R(1.0), r, u[c], v[c], w[c], cp, abl ? abl[k - 1] : R(0.0), tau[c],
-                                      false, tb);
-        if (cp.ivreman) tau[c] = tnew;
+            for (int l = 0; l < Q; ++l) fp[l] = s[l] - lat_w<Q, R>(l);
+            const MomentsT<R> m = moments<Q>(fp);
+            const R r = sc[0];
+            TurbInT<R> tb;
+            tb.on = false;
+            tb.dux = tb.duy = tb.duz = R(0);
+            const R tnew = collide<Q>(fp, m, r - R(1.0), r, sc[CELL_T], sc[2 * CELL_T], sc[3 * CELL_T], cp,
+                                      abl ? abl[a.k - 1] : R(0.0), sc[4 * CELL_T], false, tb);
+            if (cp.ivreman) tau[a.c0 + tid] = tnew;
 #pragma unroll
-        for (int l = 0; l < Q; ++l) sm[t * Q + l] = fp[l] + lat_w<Q, R>(l);
+            for (int l = 0; l < Q; ++l) s[l] = fp[l] + lat_w<Q, R>(l);
+        }
+        const bool whole = __syncthreads_and(inner);
+        tile_put<Q>(tile, f, a.c0, a.n, cells, whole);
+        __syncthreads();
     }
-    __syncthreads();
-    tile_store<Q>(sm, f, g.cell(i0, j, k), n);
 }
 
 // drift: f(l,i,j,k) = feq(l,i-cx,j-cy,k-cz) over interior cells
@@ -289,31 +334,44 @@ __global__ void __launch_bounds__(DriftTile<Q, R>::T, DriftTile<Q, R>::BLOCKS)
 
 // macrovars over the ghost-inclusive grid, summation order of m_macrovars_kernel.F90:35-49
 template <int Q, typename R = float>
-__global__ void __launch_bounds__(128) k_ref_macrovars(R* rho, R* u, R* v, R* w, const R* f,
-                                                       RefGrid g) {
-    __shared__ R sm[128 * Q];
-    const int i0 = blockIdx.x * 128, j = blockIdx.y, k = blockIdx.z;
-    const int n = min(128, g.nx + 2 - i0);
-    const int t = threadIdx.x;
-    if (n <= 0) return;
-    tile_load<Q>(sm, f, g.cell(i0, j, k), n);
-    __syncthreads();
-    if (t < n) {
-        R tr = R(0), tu = R(0), tv = R(0), tw = R(0);
+__global__ void __launch_bounds__(CELL_T, MacroTile<Q, R>::BLOCKS)
+    k_ref_macrovars(R* rho, R* u, R* v, R* w, const R* f, RefGrid g, unsigned ntiles) {
+    using P = MacroTile<Q, R>;
+    extern __shared__ __align__(16) unsigned char raw[];
+    R* sm = reinterpret_cast<R*>(raw);
+    const int tid = threadIdx.x;
+    auto fetch = [&](unsigned t, int b) {
+        const TileAt a = tile_at<true>(g, t, 0);
+        tile_fetch<Q>(sm + b * P::STAGE, f, a.c0, a.n);
+    };
+    fetch(blockIdx.x, 0);
+    cp_async_commit();
+    int b = 0;
+    for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
+        if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
+        cp_async_commit();
+        const TileAt a = tile_at<true>(g, t, 0);
+        cp_async_wait<1>();
+        __syncthreads();
+        if (tid < a.n) {
+            const R* s = sm + b * P::STAGE + phase_of(f + a.c0 * Q) + tid * Q;
+            R tr = R(0), tu = R(0), tv = R(0), tw = R(0);
 #pragma unroll
-        for (int l = 0; l < Q; ++l) {
-            const R tf = sm[t * Q + l];
-            tr = tr + tf;
-            macc(tu, lat_cx(l), tf);
-            macc(tv, lat_cy(l), tf);
-            macc(tw, lat_cz(l), tf);
+            for (int l = 0; l < Q; ++l) {
+                const R tf = s[l];
+                tr = tr + tf;
+                macc(tu, lat_cx(l), tf);
+                macc(tv, lat_cy(l), tf);
+                macc(tw, lat_cz(l), tf);
+            }
+            const R inv = R(1.0) / tr;
+            const long long c = a.c0 + tid;
+            rho[c] = tr;
+            u[c] = tu * inv;
+            v[c] = tv * inv;
+            w[c] = tw * inv;
         }
-        const R inv = R(1.0) / tr;
-        const long long c = g.cell(i0 + t, j, k);
-        rho[c] = tr;
-        u[c] = tu * inv;
-        v[c] = tv * inv;
-        w[c] = tw * inv;
+        __syncthreads();
     }
 }
 

@@ -44,3 +44,57 @@ def test_drift_moves_every_value(shape, nl, dtype):
         L.drift(f, src)
         assert torch.equal(f, want) and torch.equal(src, keep)     # ghosts and the source stay as they were
     L.close()
+
+
+def equilibrium_like(nl, shape, dtype, off, g):
+    """rho, u, v, w and an f near their equilibrium, at an alignment offset"""
+    sc = [torch.randn(shape, dtype=dtype, device="cuda", generator=g) * 0.02 for _ in range(4)]
+    sc[0] += 1.0
+    sc[1] += 0.05
+    f = at_offset(shape + (nl,), dtype, off, g)
+    w = torch.tensor([{19: (1 / 3, 1 / 18, 1 / 36, 0), 27: (8 / 27, 2 / 27, 1 / 54, 1 / 216)}[nl][sum(x * x for x in c)]
+                      for c in C[:nl]], dtype=dtype, device="cuda")
+    f.mul_(0.02).add_(1.0).mul_(w)
+    return f, sc
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("nl", [19, 27])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_postcoll_and_macrovars(shape, nl, dtype):
+    import numpy as np
+
+    from oracle import oracle as O
+    nx, ny, nz = shape
+    L = lbm_of(nx, ny, nz, nl)
+    o = O.Oracle(O.Config(nx, ny, nz, nl, iturb_pos=2), np.float64)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nx * 100 + nz)
+    s = (slice(1, -1),) * 3
+    for off in range(16 // dtype.itemsize):
+        f, sc = equilibrium_like(nl, L.p.sshape, dtype, off, g)
+        tau = torch.full(L.p.sshape, 0.5, dtype=dtype, device="cuda")
+        # macrovars: every cell, in the order of the directions, bit for bit
+        want = [torch.zeros_like(sc[0]) for _ in range(4)]
+        for l in range(nl):
+            want[0] += f[..., l]
+            for a in range(3):
+                want[a + 1] += C[l][a] * f[..., l]
+        inv = 1.0 / want[0]
+        out = [torch.full_like(sc[0], 9.0) for _ in range(4)]
+        L.macrovars(*out, f)
+        assert torch.equal(out[0], want[0]) and all(torch.equal(out[a], want[a] * inv) for a in (1, 2, 3))
+        # postcoll: the interior against the FP64 oracle, the ghosts and their tau untouched
+        before = f.clone()
+        rf, rt = (t.double().cpu().numpy().copy() for t in (f, tau))
+        o.postcoll(rf, rt, *(t.double().cpu().numpy() for t in sc))
+        L.postcoll(f, tau, *sc)
+        got, gt = f.double().cpu().numpy(), tau.double().cpu().numpy()
+        tol = 2e-6 if dtype == torch.float32 else 1e-13       # as test_gpu_percall.py: closed form against dense loops
+        assert np.linalg.norm(got[s] - rf[s]) < tol * np.linalg.norm(rf[s])
+        assert np.linalg.norm(gt[s] - rt[s]) < 100 * tol * np.linalg.norm(rt[s] - 0.5) + 1e-7 * (dtype == torch.float32) * rt[s].size ** 0.5
+        f[s] = before[s]
+        assert torch.equal(f, before)
+        tau[s] = 0.5
+        assert bool((tau == 0.5).all())
+    L.close()
