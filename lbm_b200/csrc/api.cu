@@ -623,16 +623,22 @@ const S* xg_of(const lbm_ctx* c, int b) { return c->fold ? (const S*)c->d_xg[b] 
 // after a step, periodic-j ghost rows are read as rows ny and 1 (state_kernels.cuh)
 int wrap_rows(const lbm_ctx* c) { return (c->state == ST_POST && c->p.jbnd == 0 && !c->halo_j) ? 1 : 0; }
 
+// f1 and f2 of a stepped state whose newest buffer is b
 template <int Q, typename S>
-void launch_export(lbm_ctx* c, float* ref, int b, bool pull) {
+void launch_export(lbm_ctx* c, float* f1, float* f2, int b) {
     const SoaGrid& g = c->sg;
     dim3 grd((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2);
-    if (pull)
-        k_export<Q, S, true><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], (const S*)c->buf[1 - b], ref, g,
-                                                        wrap_rows(c), xg_of<S>(c, 1 - b));
-    else
-        k_export<Q, S, false><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], nullptr, ref, g, wrap_rows(c),
-                                                         xg_of<S>(c, b));
+    k_export<Q, S, true><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], (const S*)c->buf[1 - b], f1, f2, g,
+                                                    wrap_rows(c), xg_of<S>(c, 1 - b), xg_of<S>(c, b));
+    c->launches++;
+}
+// buffer b of an imported state as it is
+template <int Q, typename S>
+void launch_export_stored(lbm_ctx* c, float* f, int b) {
+    const SoaGrid& g = c->sg;
+    dim3 grd((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2);
+    k_export<Q, S, false><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], nullptr, f, nullptr, g, wrap_rows(c),
+                                                     xg_of<S>(c, b), nullptr);
     c->launches++;
 }
 template <int Q, typename S>
@@ -1154,11 +1160,10 @@ int lbm_state_export(lbm_ctx* c, float* f1, float* f2) {
     NEED(c, f1); NEED(c, f2);
     const bool post = (c->state == ST_POST);
     if (post) {
-        DISPATCH_QS(c, launch_export, c, f1, c->cur, true);
-        DISPATCH_QS(c, launch_export, c, f2, c->cur, false);
+        DISPATCH_QS(c, launch_export, c, f1, f2, c->cur);
     } else {
-        DISPATCH_QS(c, launch_export, c, f1, c->cur, false);
-        DISPATCH_QS(c, launch_export, c, f2, 1 - c->cur, false);
+        DISPATCH_QS(c, launch_export_stored, c, f1, c->cur);
+        DISPATCH_QS(c, launch_export_stored, c, f2, 1 - c->cur);
     }
     LBM_LAUNCHED(c, "export");
     return LBM_OK;

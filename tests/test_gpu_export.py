@@ -1,0 +1,49 @@
+"""State export and macroscopic read-back in every phase of a run: chunks of a row and
+one cell past them, before the first step, after it, and into arrays of any
+alignment; the export agrees with the per-call path and writes nothing else."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("nl", [19, 27])
+@pytest.mark.parametrize("nx,ny,nz,codes", [(6, 4, 3, (1, 0, 12)), (126, 3, 4, (1, 0, 22)), (127, 4, 3, (1, 0, 11)),
+                                            (254, 3, 3, (1, 0, 12)), (20, 5, 4, (0, 0, 0)), (30, 4, 5, (0, 12, 12))])
+def test_export_matches_percall(nx, ny, nz, codes, nl, storage):
+    from lbm_b200 import Params, Solver
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nx)
+    ib, jb, kb = codes
+    p = Params(nx=nx, ny=ny, nz=nz, nl=nl, ibnd=ib, jbnd=jb, kbnd=kb, iturb_pos=2, storage=storage)
+    m = [torch.zeros(p.sshape, device="cuda") for _ in range(4)]
+    s = (slice(1, -1),) * 3
+    m[0][s] = 1.0
+    for q in (1, 2, 3):
+        m[q][s] = 0.02 * torch.randn((nz, ny, nx), device="cuda", generator=g)
+    uvel = torch.full((nz,), 0.05, device="cuda")
+    a, b = Solver(p, *m, uvel), Solver(p, *m, uvel, fused=False)
+    n = a.lbm.empty_f().numel()
+    # FP32 rounding of populations of order 0.3 over three steps; FP16 offsets keep 2^-11 of 2e-2
+    tol = 2e-6 if storage == "f32" else 1e-4
+    for step in range(3):
+        for off1, off2 in ((0, 0), (1, 2), (3, 1)):
+            pad = [torch.full((n + 8,), 7.0, device="cuda") for _ in range(2)]
+            f1, f2 = (t[o:o + n].view(p.fshape) for t, o in zip(pad, (off1, off2)))
+            a.lbm.state_export(f1, f2)
+            for x, y in zip((f1, f2), b.state()):
+                assert float((x - y).abs().max()) < tol
+            for t, o in zip(pad, (off1, off2)):
+                assert bool((t[:o] == 7.0).all()) and bool((t[o + n:] == 7.0).all())
+        e1, e2 = a.state()
+        assert torch.equal(e1, f1) and torch.equal(e2, f2)
+        for x, y in zip(a.macro(), b.macro()):
+            if step:      # before a step the ghosts of the imported moments are the caller's
+                assert float((x - y).abs().max()) < 20 * tol
+        a.step(1)
+        b.step(1)
+    # one array for both: what is left is f2, as when the arrays were written in turn
+    e1, e2 = a.state()
+    a.lbm.state_export(f1, f1)
+    assert torch.equal(f1, e2)
