@@ -331,7 +331,7 @@ void set_params_f64(lbm_ctx* c, double kinevisc, double smagorinsky, double rho0
 
 // boundarycond in the dispatch order of m_boundarycond.F90:14-468
 template <int Q, typename Acc>
-int run_bc(lbm_ctx* c, Acc f1, Acc f2, const typename Acc::real* uvel) {
+int run_bc(lbm_ctx* c, Acc f1, Acc f2, const float* uvel) {
     const int nx = c->p.nx, ny = c->p.ny, nz = c->p.nz, nl = c->p.nl;
     cudaStream_t s = c->stream;
     auto periodic = [&](int axis) {
@@ -365,10 +365,7 @@ int run_bc(lbm_ctx* c, Acc f1, Acc f2, const typename Acc::real* uvel) {
         c->launches++;
     }
     if (c->p.ibnd == 1) {
-        if constexpr (std::is_same<typename Acc::real, double>::value)
-            k_inflow<Q, Acc><<<dim3((ny + 127) / 128, nz), 128, 0, s>>>(f1, uvel, c->rho0d, c->cosdd, c->sindd);
-        else
-            k_inflow<Q, Acc><<<dim3((ny + 127) / 128, nz), 128, 0, s>>>(f1, uvel, c->p.rho0, c->cosd, c->sind);
+        k_inflow<Q, Acc><<<dim3((ny + 127) / 128, nz), 128, 0, s>>>(f1, uvel, c->p.rho0, c->cosd, c->sind);
         c->launches++;
     }
     for (int a = 0; a < 3; ++a)
@@ -377,10 +374,59 @@ int run_bc(lbm_ctx* c, Acc f1, Acc f2, const typename Acc::real* uvel) {
     return LBM_OK;
 }
 
+// the same on the reference layout.  Between the first and the second round of periodic
+// copies only the closed faces read j ghosts, and they can read them through rows ny
+// and 1 (so the first j copy, whose rows the second one writes again, is left out)
+// unless i and k are both closed: then the k faces read, through a j ghost row, an
+// x ghost that the i faces have overwritten in row ny or 1 since that copy.  Without
+// a face or an inflow in between, the second round has nothing left to do.
 template <int Q, typename R>
 int bc_ref(lbm_ctx* c, R* f1, R* f2, const R* uvel) {
-    AosAccT<R> a1{f1, c->rg}, a2{f2, c->rg};
-    return run_bc<Q>(c, a1, a2, uvel);
+    const int nx = c->p.nx, ny = c->p.ny, nz = c->p.nz;
+    cudaStream_t s = c->stream;
+    const RefGrid& g = c->rg;
+    const int codes[3] = {c->p.ibnd, c->p.jbnd, c->p.kbnd};
+    auto periodic = [&](int axis) {
+        const long long row = (long long)(nx + 2) * Q;
+        const long long n = axis == 0 ? (long long)(ny + 2) * Q : axis == 1 ? row : row * (ny + 2);
+        k_ref_periodic<R><<<dim3((unsigned)((n + 255) / 256), axis == 2 ? 1 : nz + 2), 256, 0, s>>>(f1, g, axis);
+        c->launches++;
+    };
+    const bool between = c->face_on[0] || c->face_on[1] || c->face_on[2] || c->p.ibnd == 1;
+    const bool wrap = codes[1] == 0 && between && !(c->face_on[0] && c->face_on[2]);
+    for (int a = 0; a < 3; ++a)
+        if (codes[a] == 0 && !(wrap && a == 1)) periodic(a);
+    for (int a = 0; a < 3; ++a) {
+        if (!c->face_on[a]) continue;
+        const int np = std::max(c->face[a][0].n, c->face[a][1].n);
+        const long long na = (long long)(a == 0 ? ny : nx) * np;   // threads over the first tangential extent
+        const int nb = (a == 2) ? ny : nz;
+        k_ref_closed<Q, R><<<dim3((unsigned)((na + 127) / 128), nb, 2), 128, 0, s>>>(f1, f2, g, a, c->face[a][0],
+                                                                                    c->face[a][1], wrap ? 1 : 0);
+        c->launches++;
+    }
+    AosAccT<R> a1{f1, g}, a2{f2, g};
+    for (int e = 0; e < 3; ++e) {
+        if (!c->edges_on[e]) continue;
+        const EdgeSet& es = c->edges[e];
+        k_edges<AosAccT<R>><<<dim3((es.nfree + 127) / 128, 4), 128, 0, s>>>(a1, a2, es);
+        c->launches++;
+    }
+    if (c->corners_on) {
+        k_corners<AosAccT<R>><<<1, 32, 0, s>>>(a1, a2, c->corners);
+        c->launches++;
+    }
+    if (c->p.ibnd == 1) {
+        R rho0, cosd, sind;
+        if constexpr (std::is_same<R, double>::value) { rho0 = c->rho0d; cosd = c->cosdd; sind = c->sindd; }
+        else { rho0 = c->p.rho0; cosd = c->cosd; sind = c->sind; }
+        k_ref_inflow<Q, R><<<dim3((unsigned)(((long long)ny * Q + 255) / 256), nz), 256, 0, s>>>(f1, uvel, rho0, cosd, sind, g);
+        c->launches++;
+    }
+    for (int a = 0; a < 3; ++a)
+        if (codes[a] == 0 && between) periodic(a);
+    LBM_LAUNCHED(c, "boundarycond");
+    return LBM_OK;
 }
 
 template <int Q, typename S>
@@ -794,8 +840,9 @@ int forcings_apply_run(lbm_ctx* c, R* f, const R* force, const R* rho, const R* 
 
 template <typename R>
 int solids_run(lbm_ctx* c, R* f, const int32_t* blanking) {
-    if (c->p.nl == 27) k_ref_solids<27, R><<<interior_rows(c), 128, 0, c->stream>>>(f, blanking, c->rg);
-    else k_ref_solids<19, R><<<interior_rows(c), 128, 0, c->stream>>>(f, blanking, c->rg);
+    const unsigned grd = (unsigned)((c->rg.ncell() + 3 + SOLID_CELLS - 1) / SOLID_CELLS);   // the mask's first word starts up to 3 early
+    if (c->p.nl == 27) k_ref_solids<27, R><<<grd, 256, 0, c->stream>>>(f, blanking, c->rg);
+    else k_ref_solids<19, R><<<grd, 256, 0, c->stream>>>(f, blanking, c->rg);
     c->launches++;
     LBM_LAUNCHED(c, "solids");
     return LBM_OK;

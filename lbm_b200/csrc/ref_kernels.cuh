@@ -12,6 +12,7 @@
 // points), where -r8 makes every real, tiny() and eps double precision.
 #pragma once
 
+#include "boundary.cuh"
 #include "collide.cuh"
 #include "ref_tiles.cuh"
 
@@ -442,20 +443,159 @@ __global__ void k_ref_axpy(R* f, const R* feq, long long n, int sgn) {
         f[e] = (sgn > 0) ? (feq[e] + f[e]) : (f[e] - feq[e]);
 }
 
-// solids: swap pairs (l,l+1), l = 2,4,..,nl-1 (1-based) at blanked interior cells (m_solids.F90:24-36)
+// solids: swap pairs (l,l+1), l = 2,4,..,nl-1 (1-based) at blanked interior cells (m_solids.F90:24-36).
+// A block reads 1024 mask entries in 16-byte words (its first and last ones
+// element by element), lists the blanked interior cells among them, and swaps
+// their pairs with a thread per pair, so that a cell's values move together
+// (a thread per cell walks 108 bytes by itself: 24 us for 256x128x128 with 16 boxes).
+#define SOLID_CELLS 1024
 template <int Q, typename R = float>
-__global__ void k_ref_solids(R* f, const int32_t* blank, RefGrid g) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
-    if (i > g.nx) return;
-    const long long c = g.cell(i, j, k);
-    if (blank[c] == 0) return;
-    R* p = f + c * Q;
+__global__ void __launch_bounds__(256) k_ref_solids(R* f, const int32_t* blank, RefGrid g) {
+    __shared__ int count;
+    __shared__ int list[SOLID_CELLS];
+    const long long n = g.ncell();
+    const long long e0 = (long long)blockIdx.x * SOLID_CELLS - phase_of(blank);   // first cell of the block
+    const long long e = e0 + threadIdx.x * 4;
+    if (threadIdx.x == 0) count = 0;
+    int m[4] = {0, 0, 0, 0};
+    if (e >= 0 && e + 4 <= n) {
+        const int4 q = *reinterpret_cast<const int4*>(blank + e);
+        m[0] = q.x; m[1] = q.y; m[2] = q.z; m[3] = q.w;
+    } else {
 #pragma unroll
-    for (int l = 1; l + 1 < Q; l += 2) {
-        const R a = p[l];
-        p[l] = p[l + 1];
-        p[l + 1] = a;
+        for (int v = 0; v < 4; ++v)
+            if (e + v >= 0 && e + v < n) m[v] = blank[e + v];
     }
+    if (!__syncthreads_or(m[0] | m[1] | m[2] | m[3])) return;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        if (m[v] == 0) continue;
+        const long long c = e + v, row = c / (g.nx + 2), k = row / (g.ny + 2);
+        const int i = (int)(c - row * (g.nx + 2)), j = (int)(row - k * (g.ny + 2));
+        if (i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz)
+            list[atomicAdd(&count, 1)] = threadIdx.x * 4 + v;
+    }
+    __syncthreads();
+    constexpr int NP = Q / 2;
+    const int work = count * NP;
+    for (int w = threadIdx.x; w < work; w += 256) {
+        const int cell = w / NP, q = w - cell * NP;
+        R* p = f + (e0 + list[cell]) * Q + 1 + 2 * q;
+        const R x = p[0], y = p[1];
+        p[0] = y;
+        p[1] = x;
+    }
+}
+
+// ---- boundarycond on the reference layout ------------------------------------------
+// The kernels of boundary.cuh give a thread a cell (or one direction of cells that
+// lie nl elements apart), which suits a structure of arrays.  Here l is fastest,
+// so consecutive threads take consecutive directions of a cell.
+
+// the periodic copies of one axis (m_boundary_{i,j,k}_periodic_kernel.F90): the
+// ghost planes 0 and n+1 from the planes n and 1.  A thread per element of a
+// plane's contiguous pieces (axis 0: a cell, 1: a row, 2: the whole plane).
+// Grid: x over a piece's elements (axis 0: over the rows' cells), y over the planes k.
+template <typename R>
+__global__ void __launch_bounds__(256) k_ref_periodic(R* __restrict__ f, RefGrid g, int axis) {
+    const long long row = (long long)(g.nx + 2) * g.nl, plane = row * (g.ny + 2);
+    const long long e = (long long)blockIdx.x * 256 + threadIdx.x;
+    long long at, step;
+    int n;
+    if (axis == 0) {
+        const long long j = e / g.nl;
+        if (j > g.ny + 1) return;
+        at = j * row + (e - j * g.nl) + blockIdx.y * plane;
+        step = g.nl;
+        n = g.nx;
+    } else if (axis == 1) {
+        if (e >= row) return;
+        at = e + blockIdx.y * plane;
+        step = row;
+        n = g.ny;
+    } else {
+        if (e >= plane) return;
+        at = e;
+        step = plane;
+        n = g.nz;
+    }
+    R* p = f + at;
+    const R lo = p[n * step], hi = p[step];
+    p[0] = lo;
+    p[(n + 1) * step] = hi;
+}
+
+// closed faces of one axis, both sides in one launch (blockIdx.z = side): k_closed of
+// boundary.cuh with a thread per (outgoing direction, cell).  wrap (periodic j):
+// a source row 0 or ny+1 is read as row ny or 1, so the periodic j copy that
+// comes before it in m_boundarycond.F90 need not run.
+template <int Q, typename R>
+__global__ void __launch_bounds__(128) k_ref_closed(R* f1, const R* f2, RefGrid g, int axis, FacePairs lo, FacePairs hi, int wrap) {
+    __shared__ int8_t tl[9], tm[9], tc[9][3];
+    const int side = blockIdx.z;
+    if (threadIdx.x < 9) {
+        const FacePairs& fp = side ? hi : lo;
+        const int q = threadIdx.x;
+        tl[q] = fp.l[q];
+        tm[q] = fp.m[q];
+        tc[q][0] = fp.cx[q];
+        tc[q][1] = fp.cy[q];
+        tc[q][2] = fp.cz[q];
+    }
+    __syncthreads();
+    const int np = side ? hi.n : lo.n;
+    const int e = blockIdx.x * 128 + threadIdx.x;
+    const int a = e / np + 1, q = e - (a - 1) * np;         // first tangential index, pair
+    const int b = blockIdx.y + 1;
+    int x[3];
+    if (axis == 0) {
+        if (a > g.ny) return;
+        x[0] = side ? g.nx + 1 : 0; x[1] = a; x[2] = b;
+    } else if (axis == 1) {
+        if (a > g.nx) return;
+        x[0] = a; x[1] = side ? g.ny + 1 : 0; x[2] = b;
+    } else {
+        if (a > g.nx) return;
+        x[0] = a; x[1] = b; x[2] = side ? g.nz + 1 : 0;
+    }
+    const int l = tl[q], m = tm[q];
+    // source: the plane next to the ghost, shifted by -c in the tangential directions
+    const int n[3] = {g.nx, g.ny, g.nz};
+    int s[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = (d == axis) ? (side ? n[d] : 1) : x[d] - tc[q][d];
+    if (wrap) s[1] = s[1] == 0 ? g.ny : (s[1] == g.ny + 1 ? 1 : s[1]);
+    const long long o = g.cell(x[0], x[1], x[2]) * Q;
+    const R refl = f2[o + l], out = f1[g.cell(s[0], s[1], s[2]) * Q + l];
+    f1[o + m] = refl;
+    f1[o + l] = out;
+}
+
+// inflow at i = 0 and zero-gradient outflow at i = nx+1: k_inflow of boundary.cuh with a
+// thread per (direction, j); grid y over k
+template <int Q, typename R>
+__global__ void __launch_bounds__(256) k_ref_inflow(R* __restrict__ f, const R* __restrict__ uvel, R rho0, R cosd, R sind, RefGrid g) {
+    __shared__ R tw[Q], tx[Q], ty[Q];
+    __shared__ int ts[Q];
+    if (threadIdx.x < Q) {
+        const int l = threadIdx.x;
+        const int s = lat_cx(l) > 0 ? lat_opposite(l) : l;   // the direction whose corrected value goes to ghost l
+        ts[l] = s;
+        tw[l] = lat_w<Q, R>(s);
+        tx[l] = (R)lat_cx(s);
+        ty[l] = (R)lat_cy(s);
+    }
+    __syncthreads();
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    const int j = e / Q + 1, l = e - (j - 1) * Q, k = blockIdx.y + 1;
+    if (j > g.ny) return;
+    R* row = f + g.cell(0, j, k) * Q;
+    const R uu = uvel[k - 1];
+    const R cs2 = R(1) / R(3);
+    const R in = row[Q + ts[l]] - R(2) * tw[l] * rho0 * (tx[l] * uu * cosd + ty[l] * uu * sind) / cs2;
+    const R out = row[(long long)g.nx * Q + l];
+    row[l] = in;
+    row[(long long)(g.nx + 1) * Q + l] = out;
 }
 
 // forcings_apply: f += feq2(rho, u - F/rho) - feq2(rho, u) at interior cells with
