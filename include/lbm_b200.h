@@ -64,7 +64,7 @@ enum {
 enum {
     LBM_KERNEL_PULL = 1,   /* direct coalesced global loads, one cell per thread              */
     LBM_KERNEL_PAIR = 2    /* (default) two cells per thread on the packed f32x2 pipes; needs
-                              ihrr=1, even nx >= 4 (other cases run LBM_KERNEL_PULL)          */
+                              ihrr=1, nx >= 4 (other cases run LBM_KERNEL_PULL)               */
 };
 
 /* Run-time options.  Field meanings follow m_readinfile.F90:3-58 and

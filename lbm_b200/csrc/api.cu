@@ -512,15 +512,16 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// the two-cells-per-thread kernel (pair_step.cuh) covers the regularized collision on even nx, at any
-// state size (64-bit byte offsets)
-bool pair_shape_ok(const lbm_ctx* c) { return c->p.ihrr == 1 && c->p.nx % 2 == 0 && c->p.nx >= 4; }
-bool pair_ok(const lbm_ctx* c) { return c->kernel == LBM_KERNEL_PAIR && pair_shape_ok(c); }
-dim3 pair_grid(const lbm_ctx* c, int t) { return dim3((unsigned)((c->p.nx / 2 + t - 1) / t), c->p.ny, c->p.nz); }
+// the two-cells-per-thread kernel (pair_step.cuh) covers the regularized collision at any state size
+// (64-bit byte offsets); the external forcing and the j-slab tiles in the folded configuration take
+// an even nx only
+bool pair_ok(const lbm_ctx* c) { return c->kernel == LBM_KERNEL_PAIR && c->p.ihrr == 1 && c->p.nx >= 4; }
+bool pair_even_ok(const lbm_ctx* c) { return pair_ok(c) && c->p.nx % 2 == 0; }
 
-template <int Q, typename S, bool WRAP, bool FORCE, bool FOLD, int T>
+template <int Q, typename S, bool WRAP, bool FORCE, bool FOLD, int T, bool ODD = false>
 cudaError_t pair_launch(lbm_ctx* c, const S* src, S* dst, const StepArgs& a) {
-    return launch_pdl(k_step_pair<Q, S, WRAP, FORCE, FOLD, T>, pair_grid(c, T), dim3(T), c->stream, src, dst, a);
+    const dim3 grd((unsigned)(((c->p.nx + 1) / 2 + T - 1) / T), c->p.ny, c->p.nz);
+    return launch_pdl(k_step_pair<Q, S, WRAP, FORCE, FOLD, T, ODD>, grd, dim3(T), c->stream, src, dst, a);
 }
 
 // the steady step from buffer cur into nxt, two cells per thread
@@ -528,15 +529,28 @@ template <int Q, typename S, bool WRAP, bool FOLD>
 int pair_family_step(lbm_ctx* c, int nxt, const StepArgs& a) {
     const S* src = (const S*)c->buf[c->cur];
     S* dst = (S*)c->buf[nxt];
-    // blocks of 256 threads where that shape is compiled and a row's pairs fill them
-    const bool wide = pair_wide_ok<Q, S>() && (c->p.nx / 2) % 256 == 0;
+    const int t = pair_width<Q, S>((c->p.nx + 1) / 2);
+    constexpr int W = (sizeof(S) == 2 && Q == 27) ? 256 : 128;
     cudaError_t r;
-    if (c->force)
-        r = wide ? pair_launch<Q, S, WRAP, true, FOLD, pair_wide_ok<Q, S>() ? 256 : 128>(c, src, dst, a)
-                 : pair_launch<Q, S, WRAP, true, FOLD, 128>(c, src, dst, a);
-    else
-        r = wide ? pair_launch<Q, S, WRAP, false, FOLD, pair_wide_ok<Q, S>() ? 256 : 128>(c, src, dst, a)
-                 : pair_launch<Q, S, WRAP, false, FOLD, 128>(c, src, dst, a);
+    if (c->p.nx % 2 != 0) {
+        // callers have checked that an odd nx has no forcing and no slab tile here
+        if constexpr (WRAP == FOLD)
+            r = t < 128 ? pair_launch<Q, S, WRAP, false, FOLD, 32, true>(c, src, dst, a)
+                        : pair_launch<Q, S, WRAP, false, FOLD, 128, true>(c, src, dst, a);
+        else
+            r = cudaErrorInvalidValue;
+    } else if (c->force) {
+        r = t == 256 ? pair_launch<Q, S, WRAP, true, FOLD, W>(c, src, dst, a)
+                     : pair_launch<Q, S, WRAP, true, FOLD, 128>(c, src, dst, a);
+    } else if (t == 256) {
+        r = pair_launch<Q, S, WRAP, false, FOLD, W>(c, src, dst, a);
+    } else if (t == 128) {
+        r = pair_launch<Q, S, WRAP, false, FOLD, 128>(c, src, dst, a);
+    } else if (t == 64) {
+        r = pair_launch<Q, S, WRAP, false, FOLD, 64>(c, src, dst, a);
+    } else {
+        r = pair_launch<Q, S, WRAP, false, FOLD, 32>(c, src, dst, a);
+    }
     LBM_TRY(cuda_check(c, r, "fused step (pair)"));
     c->launches++;
     LBM_LAUNCHED(c, "fused step (pair)");
@@ -545,7 +559,7 @@ int pair_family_step(lbm_ctx* c, int nxt, const StepArgs& a) {
 
 template <int Q, typename S>
 int step_one(lbm_ctx* c) {
-    if (c->force && !pair_ok(c))
+    if (c->force && !pair_even_ok(c))
         return fail(c, LBM_ERR_UNSUPPORTED, "step: the fused external forcing runs in the two-cells-per-thread kernel "
                                             "(LBM_KERNEL_PAIR, ihrr = 1, even nx >= 4); use lbm_forcings_apply per call");
     const SoaGrid& g = c->sg;
@@ -568,7 +582,7 @@ int step_one(lbm_ctx* c) {
         LBM_TRY(prof_begin(c));
         if (c->halo_j) {
             // a j-slab tile: pull the stored halo planes, keep the folded boundaries
-            if (!pair_ok(c))
+            if (!pair_even_ok(c))
                 return fail(c, LBM_ERR_UNSUPPORTED, "step: a j-slab tile in the folded configuration runs the "
                                                     "two-cells-per-thread kernel (LBM_KERNEL_PAIR, ihrr = 1, even nx >= 4)");
             LBM_TRY((pair_family_step<Q, S, false, true>(c, nxt, a)));

@@ -12,7 +12,9 @@
 //
 // Layout facts this relies on: interior i = 1 sits at an even element of its
 // row, the row pitch and the direction stride are even, so the first cell of a
-// pair is 8-byte (FP32) / 4-byte (FP16) aligned; nx is even.
+// pair is 8-byte (FP32) / 4-byte (FP16) aligned.  With an odd nx (ODD) the last
+// pair of a row is (nx, nx+1): its second lane computes on the x ghost and the
+// row's padding, raises no flag and is not stored.
 #pragma once
 
 #include "state_kernels.cuh"
@@ -304,7 +306,7 @@ struct SepArraySink {
 // return fp holds the post-collision offsets (times store_scale<S>()).  (Variants
 // that moved the turbulence slice out of the step kernel -- a one-cell post-pass,
 // or a captured FP32 copy finished by a second kernel -- measured slower on B200.)
-template <int Q, typename S, bool FORCE = false>
+template <int Q, typename S, bool FORCE = false, bool ODD = false>
 __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int i, int j, int k) {
     Moments2 m = moments_rows2<Q>(fp);
     if constexpr (sizeof(S) == 2) {
@@ -317,9 +319,18 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
     const f2 rho = add2(bc2(1.0f), m.s0);
     const f2 inv = rcp2<S>(rho);
     const f2 ux = mul2(m.jx, inv), uy = mul2(m.jy, inv), uz = mul2(m.jz, inv);
-    flag_bad_density2(a.status, rho, add2(add2(rho, ux), add2(uy, uz)));
+    const f2 chk = add2(add2(rho, ux), add2(uy, uz));
+    const bool tail = ODD && i == a.g.nx;
+    flag_bad_density2(a.status, tail ? make_float2(rho.x, rho.x) : rho, tail ? make_float2(chk.x, chk.x) : chk);
     bool solid0 = false, solid1 = false;
-    if (a.solid) {
+    if (ODD) {
+        // rows of the mask start at any byte
+        if (a.solid) {
+            const uint8_t* s = a.solid + ((long long)(k - 1) * a.g.ny + (j - 1)) * a.g.nx + (i - 1);
+            solid0 = s[0] != 0;
+            solid1 = !tail && s[1] != 0;
+        }
+    } else if (a.solid) {
         const unsigned short s2 =
             *reinterpret_cast<const unsigned short*>(a.solid + ((long long)(k - 1) * a.g.ny + (j - 1)) * a.g.nx + (i - 1));
         solid0 = (s2 & 0xffu) != 0;
@@ -394,13 +405,13 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
 
 // The edge copy of the folded boundaries: the post-collision populations of the
 // pair holding i = 1 or i = nx, into the compact edge array.
-template <int Q, typename S>
+template <int Q, typename S, bool ODD = false>
 __device__ __forceinline__ void pair_edge(const f2 (&fp)[Q], const StepArgs& a, int i, int j, int k) {
-    if (i == 1 || i + 1 == a.g.nx) {
+    if (i == 1 || (ODD ? i : i + 1) == a.g.nx) {
         // the boundary kernel builds the inflow/outflow ghosts from these, read coalesced
         const long long nyz = (long long)a.g.ny * a.g.nz;
-        const int c = (i == 1) ? 0 : 1;
-        S* e = (S*)a.edge + (long long)c * Q * nyz + (long long)(k - 1) * a.g.ny + (j - 1);
+        const int side = (i == 1) ? 0 : 1, c = ODD ? 0 : side;
+        S* e = (S*)a.edge + (long long)side * Q * nyz + (long long)(k - 1) * a.g.ny + (j - 1);
 #pragma unroll
         for (int l = 0; l < Q; ++l) {
             if constexpr (sizeof(S) == 2) e[l * nyz] = __float2half_rn(comp(fp[l], c));   // already 2^8-scaled
@@ -411,11 +422,22 @@ __device__ __forceinline__ void pair_edge(const f2 (&fp)[Q], const StepArgs& a, 
 
 // Everything after the loads of one pair: pair_collide, the stores and the edge
 // copy of the folded boundaries (FOLD).
-template <int Q, typename S, bool FOLD, bool FORCE = false>
+template <int Q, typename S, bool FOLD, bool FORCE = false, bool ODD = false>
 __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, const StepArgs& a, long long o, int i,
                                             int j, int k) {
-    pair_collide<Q, S, FORCE>(fp, a, i, j, k);
+    pair_collide<Q, S, FORCE, ODD>(fp, a, i, j, k);
     S* q = dst + o;
+    if (ODD && i == a.g.nx) {
+        // one cell is left of the row
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+            S* p = reinterpret_cast<S*>(reinterpret_cast<char*>(q) + a.soffb[l]);
+            if constexpr (sizeof(S) == 2) *p = __float2half_rn(fp[l].x);
+            else *p = fp[l].x;
+        }
+        if (FOLD) pair_edge<Q, S, ODD>(fp, a, i, j, k);
+        return;
+    }
     if constexpr (sizeof(S) == 2) {
         // the edge copy reuses the stored half2 values (no second conversion)
         __half2 h[Q];
@@ -424,7 +446,7 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
             h[l] = __floats2half2_rn(fp[l].x, fp[l].y);
             *reinterpret_cast<__half2*>(reinterpret_cast<char*>(q) + a.soffb[l]) = h[l];
         }
-        if (FOLD && (i == 1 || i + 1 == a.g.nx)) {
+        if (FOLD && (i == 1 || (!ODD && i + 1 == a.g.nx))) {
             const long long nyz = (long long)a.g.ny * a.g.nz;
             const int c = (i == 1) ? 0 : 1;
             __half* e = (__half*)a.edge + (long long)c * Q * nyz + (long long)(k - 1) * a.g.ny + (j - 1);
@@ -434,7 +456,7 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
     } else {
 #pragma unroll
         for (int l = 0; l < Q; ++l) *reinterpret_cast<float2*>(reinterpret_cast<char*>(q) + a.soffb[l]) = fp[l];
-        if (FOLD) pair_edge<Q, S>(fp, a, i, j, k);
+        if (FOLD) pair_edge<Q, S, ODD>(fp, a, i, j, k);
     }
 }
 
@@ -442,7 +464,7 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
 // j read through rows ny and 1; FOLD: the folded boundaries follow (edge copy).
 // A j-slab tile in the folded configuration pulls its stored halo planes
 // (WRAP false) and keeps the folded boundaries (FOLD true).
-template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP>
+template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, bool ODD = false>
 __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restrict__ dst, const StepArgs& a, int i, int j,
                                           int k) {
     const long long o = a.g.off(i, j, k);
@@ -454,7 +476,7 @@ __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restri
         const S* pym = (WRAP && j == a.g.ny) ? p0 - wrapd : p0;
         PairLoad<Q, S, 0>::run(fp, p0, pyp, pym, a);
     }
-    pair_update<Q, S, FOLD, FORCE>(fp, dst, a, o, i, j, k);
+    pair_update<Q, S, FOLD, FORCE, ODD>(fp, dst, a, o, i, j, k);
 }
 
 #ifndef LBM_PAIR_MIN_BLOCKS
@@ -470,23 +492,34 @@ __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restri
 #ifndef LBM_PAIR_MIN_BLOCKS16_19
 #define LBM_PAIR_MIN_BLOCKS16_19 7
 #endif
-// the wide block of 256 threads: FP16 D3Q27 only
-template <int Q, typename S>
-__host__ __device__ constexpr bool pair_wide_ok() { return sizeof(S) == 2 && Q == 27; }
-// minimum resident blocks per SM for T threads per block (the register cap)
+// minimum resident blocks per SM for T threads per block (the register cap; an SM holds
+// 32 blocks)
 template <int Q, typename S, int T>
 __host__ __device__ constexpr int pair_min_blocks() {
-    return sizeof(S) == 2 ? (Q == 27 ? LBM_PAIR_MIN_BLOCKS16_27 * 128 / T : LBM_PAIR_MIN_BLOCKS16_19) : LBM_PAIR_MIN_BLOCKS;
+    return (sizeof(S) == 2 ? (Q == 27 ? LBM_PAIR_MIN_BLOCKS16_27 : LBM_PAIR_MIN_BLOCKS16_19) : LBM_PAIR_MIN_BLOCKS) * 128 / T;
 }
-// Grid: x covers nx/2 pairs in blocks of T threads, y = j, z = k.  Needs
-// ihrr = 1 and nx even; offsets are 64-bit, so any state size.
-template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, int T = 128>
+// Threads per block for rows of hp pairs: the width among those compiled that
+// leaves the fewest threads idle at the row's end, the widest of equals (a row of
+// 64 pairs leaves half of a block of 128 idle: D3Q27 FP32 128x64x64 29.9 us in blocks
+// of 128, 27.5 in blocks of 64; 40x32x24, 20 pairs a row, 7.2 and 5.2 in blocks of
+// 32).  256 threads are compiled for FP16 D3Q27 only and taken where they fill.
+template <int Q, typename S>
+inline int pair_width(int hp) {
+    if (sizeof(S) == 2 && Q == 27 && hp % 256 == 0) return 256;
+    int best = 128;
+    for (int t = 64; t >= 32; t /= 2)
+        if ((hp + t - 1) / t * t < (hp + best - 1) / best * best) best = t;
+    return best;
+}
+// Grid: x covers the row's pairs in blocks of T threads, y = j, z = k.  Needs
+// ihrr = 1 (and an even nx without ODD); offsets are 64-bit, so any state size.
+template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, int T = 128, bool ODD = false>
 __global__ void __launch_bounds__(T, pair_min_blocks<Q, S, T>()) k_step_pair(const S* __restrict__ src, S* __restrict__ dst,
                                                                              StepArgs a) {
     pdl_enter();
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + 1;
     if (i > a.g.nx) return;
-    pair_cell<Q, S, WRAP, FORCE, FOLD>(src, dst, a, i, blockIdx.y + 1, blockIdx.z + 1);
+    pair_cell<Q, S, WRAP, FORCE, FOLD, ODD>(src, dst, a, i, blockIdx.y + 1, blockIdx.z + 1);
 }
 
 }  // namespace lbm
