@@ -435,6 +435,11 @@ int bc_state(lbm_ctx* c, int i1, int i2) {
     return run_bc<Q>(c, a1, a2, c->d_uvel);
 }
 
+// periodic in every direction (the surface's cells fit 32-bit indices)
+bool periodic_box(const lbm_ctx* c) {
+    return c->p.ibnd == 0 && c->p.jbnd == 0 && c->p.kbnd == 0 && ghost_cells(c->sg) < (1LL << 31) - 128;
+}
+
 StepArgs step_args(lbm_ctx* c) {
     StepArgs a;
     memset(&a, 0, sizeof(a));
@@ -466,6 +471,7 @@ StepArgs step_args(lbm_ctx* c) {
     a.sind = c->sind;
     a.d_it_rw = c->d_it;
     a.edge = c->d_edge;
+    a.peri = periodic_box(c) ? 1 : 0;
     a.full_sector = (c->p.nx % (32 / (int)c->elem)) == 0;
     a.xg_dst = c->d_xg[1 - c->cur];
     a.force = c->force;
@@ -624,11 +630,21 @@ int step_one(lbm_ctx* c) {
         timed = true;
         c->cur = nxt;
     }
-    LBM_TRY(bc_state<Q, S>(c, c->cur, 1 - c->cur));
-    if (c->fold) launch_gather_xg<Q, S>(c, c->cur);
-    k_bump_step<<<1, 32, 0, c->stream>>>(c->d_it);
-    c->launches++;
-    LBM_LAUNCHED(c, "step counter");
+    if (periodic_box(c)) {
+        // after the pair kernel the i ghosts of the interior rows are there already
+        const bool irows = !(timed && pair_ok(c));
+        const long long n = ghost_cells(g) - (irows ? 0 : 2LL * g.ny * g.nz);
+        LBM_TRY(cuda_check(c, launch_pdl(k_periodic_all<Q, S>, dim3((unsigned)((n + 127) / 128)), dim3(128), c->stream,
+                                         (S*)c->buf[c->cur], g, c->d_it, irows ? 1 : 0), "periodic boundaries"));
+        c->launches++;
+        LBM_LAUNCHED(c, "periodic boundaries");
+    } else {
+        LBM_TRY(bc_state<Q, S>(c, c->cur, 1 - c->cur));
+        if (c->fold) launch_gather_xg<Q, S>(c, c->cur);
+        k_bump_step<<<1, 32, 0, c->stream>>>(c->d_it);
+        c->launches++;
+        LBM_LAUNCHED(c, "step counter");
+    }
     if (timed) LBM_TRY(prof_bound(c));   // the boundaries of a timed step
     c->it += 1;
     return LBM_OK;

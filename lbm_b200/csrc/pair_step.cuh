@@ -427,6 +427,22 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
                                             int j, int k) {
     pair_collide<Q, S, FORCE, ODD>(fp, a, i, j, k);
     S* q = dst + o;
+    if (!FOLD && a.peri && (i == 1 || i + 2 > a.g.nx)) {
+        // periodic i: the ghosts nx+1 and 0 of this row from the cells 1 and nx
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+            S* p = reinterpret_cast<S*>(reinterpret_cast<char*>(q) + a.soffb[l]);
+            const float hi = (ODD && i == a.g.nx) ? fp[l].x : fp[l].y;
+            const int at = (ODD && i == a.g.nx) ? -a.g.nx : 1 - a.g.nx;
+            if constexpr (sizeof(S) == 2) {
+                if (i == 1) p[a.g.nx] = __float2half_rn(fp[l].x);
+                if (i + 2 > a.g.nx) p[at] = __float2half_rn(hi);
+            } else {
+                if (i == 1) p[a.g.nx] = fp[l].x;
+                if (i + 2 > a.g.nx) p[at] = hi;
+            }
+        }
+    }
     if (ODD && i == a.g.nx) {
         // one cell is left of the row
 #pragma unroll

@@ -75,6 +75,7 @@ struct alignas(16) StepArgs {
     float rho0, cosd, sind;   // inflow constants (m_boundary_i_inflow_kernel.F90:35,71-73)
     int* d_it_rw;             // step counter, advanced by the boundary kernel
     void* edge;               // post-collision populations at i=1 and i=nx: [side][l][k-1][j-1]
+    int peri;                 // periodic in i, j and k: the pair kernel writes the i ghosts
     int full_sector;          // x-ghost sectors hold nothing but the ghost and padding
     void* xg_dst;             // x-ghost columns of the buffer the step writes: [side][l][k-1][j-1]
     const float* force;       // external_forcing(3,0:nx+1,0:ny+1,0:nz+1) or null (pair kernel only)
@@ -424,6 +425,49 @@ __device__ __forceinline__ bool ghost_cell(const SoaGrid& g, long long t, int& i
 }
 inline long long ghost_cells(const SoaGrid& g) {
     return (2LL * (g.ny + 2) + 2LL * g.nz) * (g.nx + 2) + 2LL * g.ny * g.nz;
+}
+
+// boundarycond of a domain periodic in i, j and k: after the reference's copies, axis
+// by axis (m_boundarycond.F90:21-59), a ghost cell holds the interior cell its
+// indices wrap to, so a thread per ghost cell copies that cell's values, all
+// axes in one launch, loads before stores.  Also advances the step counter.
+// irows: also the i ghosts of the interior rows, which the pair kernel writes
+// itself from registers (StepArgs::peri; a sector per value here, 35 of 127 us a
+// step for D3Q19 201x150x97).
+template <int Q, typename T>
+__global__ void __launch_bounds__(128) k_periodic_all(T* __restrict__ f, SoaGrid g, int* d_it, int irows) {
+    pdl_enter();
+    const int t = blockIdx.x * 128 + threadIdx.x;
+    if (t == 0) *d_it += 1;
+    const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const int w = nx + 2, nfull = (2 * (ny + 2) + 2 * nz) * w;   // ghost_cell's numbering in 32 bits
+    int i, j, k;
+    if (t < nfull) {
+        const int r = t / w;
+        i = t - r * w;
+        if (r < 2 * (ny + 2)) {
+            k = r < ny + 2 ? 0 : nz + 1;
+            j = r < ny + 2 ? r : r - (ny + 2);
+        } else {
+            const int q = r - 2 * (ny + 2);
+            j = q < nz ? 0 : ny + 1;
+            k = 1 + (q < nz ? q : q - nz);
+        }
+    } else {
+        const int u = t - nfull;
+        if (!irows || u >= 2 * ny * nz) return;
+        i = (u & 1) ? nx + 1 : 0;
+        k = (u >> 1) / ny;
+        j = 1 + (u >> 1) - k * ny;
+        ++k;
+    }
+    const long long o = g.off(i, j, k);
+    const long long s = g.off(wrapj(i, nx), wrapj(j, ny), wrapj(k, nz));
+    T v[Q];
+#pragma unroll
+    for (int l = 0; l < Q; ++l) v[l] = f[(long long)l * g.dstride + s];
+#pragma unroll
+    for (int l = 0; l < Q; ++l) f[(long long)l * g.dstride + o] = v[l];
 }
 
 // Copy every ghost entry (all directions) of one state buffer to another: the
