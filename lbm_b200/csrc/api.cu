@@ -1467,30 +1467,35 @@ int lbm_halo_plane_bytes(lbm_ctx* c, int64_t* bytes) {
     return LBM_OK;
 }
 
-static int halo_plane(lbm_ctx* c, void* buf, int j, bool unpack) {
-    const long long n = (long long)c->p.nl * (c->p.nz + 2) * (c->p.nx + 2);
-    const unsigned grd = (unsigned)((n + 255) / 256);
+// both planes of a tile: rows jlo, jhi to or from the arrays lo, hi (null: that one stays)
+static void halo_planes(lbm_ctx* c, void* lo, void* hi, int jlo, int jhi, bool unpack) {
     const int Q = c->p.nl;
+    const long long per = (long long)(c->p.nz + 2) * (c->p.nx + 2);   // elements of a direction
+    const int most = (int)std::max(1LL, std::min<long long>(Q, ((1LL << 31) - 256) / per));
+    const FastDiv row = make_fastdiv((unsigned)(c->p.nx + 2)), col = make_fastdiv((unsigned)(c->p.nz + 2));
     void* f = c->buf[c->cur];
     // folded configuration after a step: the x ghosts of every direction are in the compact array
-    const void* xg = (c->fold && c->state == ST_POST) ? c->d_xg[c->cur] : nullptr;
-    if (c->elem == 2) {
-        if (unpack) k_halo_plane<uint16_t, true><<<grd, 256, 0, c->stream>>>((uint16_t*)buf, (uint16_t*)f, c->sg, j, Q, nullptr);
-        else k_halo_plane<uint16_t, false><<<grd, 256, 0, c->stream>>>((uint16_t*)buf, (uint16_t*)f, c->sg, j, Q, (const uint16_t*)xg);
-    } else {
-        if (unpack) k_halo_plane<uint32_t, true><<<grd, 256, 0, c->stream>>>((uint32_t*)buf, (uint32_t*)f, c->sg, j, Q, nullptr);
-        else k_halo_plane<uint32_t, false><<<grd, 256, 0, c->stream>>>((uint32_t*)buf, (uint32_t*)f, c->sg, j, Q, (const uint32_t*)xg);
+    const void* xg = (!unpack && c->fold && c->state == ST_POST) ? c->d_xg[c->cur] : nullptr;
+    auto run = [&](auto t, int l0, int nl) {
+        using T = decltype(t);
+        const dim3 grd((unsigned)((nl * per + 255) / 256), 2);
+        if (unpack)
+            k_halo_planes<T, true><<<grd, 256, 0, c->stream>>>((T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
+        else
+            k_halo_planes<T, false><<<grd, 256, 0, c->stream>>>((T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
+        c->launches++;
+    };
+    for (int l0 = 0; l0 < Q; l0 += most) {
+        const int nl = std::min(most, Q - l0);
+        if (c->elem == 2) run(uint16_t{}, l0, nl); else run(uint32_t{}, l0, nl);
     }
-    c->launches++;
-    return LBM_OK;
 }
 
 int lbm_halo_pack_j(lbm_ctx* c, void* to_south, void* to_north) {
     if (!c) return LBM_ERR_ARG;
     if (!c->halo_j) return fail(c, LBM_ERR_STATE, "halo_pack_j: lbm_set_halo_j(ctx, 1) was not called");
     if (c->state == ST_NONE) return fail(c, LBM_ERR_STATE, "halo_pack_j: no state imported");
-    if (to_south) halo_plane(c, to_south, 1, false);
-    if (to_north) halo_plane(c, to_north, c->p.ny, false);
+    if (to_south || to_north) halo_planes(c, to_south, to_north, 1, c->p.ny, false);
     LBM_LAUNCHED(c, "halo pack");
     return LBM_OK;
 }
@@ -1499,8 +1504,8 @@ int lbm_halo_unpack_j(lbm_ctx* c, const void* from_south, const void* from_north
     if (!c) return LBM_ERR_ARG;
     if (!c->halo_j) return fail(c, LBM_ERR_STATE, "halo_unpack_j: lbm_set_halo_j(ctx, 1) was not called");
     if (c->state == ST_NONE) return fail(c, LBM_ERR_STATE, "halo_unpack_j: no state imported");
-    if (from_south) halo_plane(c, const_cast<void*>(from_south), 0, true);
-    if (from_north) halo_plane(c, const_cast<void*>(from_north), c->p.ny + 1, true);
+    if (from_south || from_north)
+        halo_planes(c, const_cast<void*>(from_south), const_cast<void*>(from_north), 0, c->p.ny + 1, true);
     LBM_LAUNCHED(c, "halo unpack");
     return LBM_OK;
 }

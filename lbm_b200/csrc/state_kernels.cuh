@@ -515,23 +515,26 @@ inline long long fold_ghost_cells(const SoaGrid& g) {
     return 2LL * g.ny * (g.nx + 2) + 2LL * ((g.nz > 1) ? 2 : 1) * g.ny;
 }
 
-// Plane j of a state buffer (every i = 0..nx+1, k = 0..nz+1 and direction) to or
-// from a contiguous array buf[l][k][i]: the halo planes of a j slab.  UNPACK:
-// buf -> buffer.  xg (packing, folded configuration): the compact x-ghost array
-// of the buffer, which holds every direction of the x ghosts of rows 1..ny (the
-// rows hold only the pulled ones).  One thread per element of buf, flat (the
-// plane is 2 KB row segments spread over the whole buffer; more elements per
-// thread measured no faster).
+// Planes jlo and jhi of a state buffer (every i = 0..nx+1, k = 0..nz+1 and direction)
+// to or from contiguous arrays blo, bhi [l][k][i] (either may be null): the halo
+// planes of a j slab.  UNPACK: arrays -> buffer.  xg (packing, folded
+// configuration): the compact x-ghost array of the buffer, which holds every
+// direction of the x ghosts of rows 1..ny (the rows hold only the pulled ones).
+// One thread per element, flat (the planes are 2 KB row segments spread over the
+// whole buffer; more elements per thread measured no faster), both planes in
+// one launch (blockIdx.y).  row, col: division by the row length nx + 2 and by
+// nz + 2; l0, nl: the directions of this launch, fewer than 2^31 elements.
 template <typename T, bool UNPACK>
-__global__ void __launch_bounds__(256) k_halo_plane(T* buf, T* f, SoaGrid g, int j, int Q, const T* __restrict__ xg) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int w = g.nx + 2;
-    const long long n = (long long)Q * (g.nz + 2) * w;
-    if (q >= n) return;
-    const long long r = q / w;
-    const int i = (int)(q - r * w);
-    const int k = (int)(r % (g.nz + 2)), l = (int)(r / (g.nz + 2));
+__global__ void __launch_bounds__(256) k_halo_planes(T* blo, T* bhi, T* f, SoaGrid g, int jlo, int jhi, int Q,
+                                                     const T* __restrict__ xg, FastDiv row, FastDiv col, int l0, int nl) {
+    T* buf = blockIdx.y ? bhi : blo;
+    const int j = blockIdx.y ? jhi : jlo;
+    const unsigned q = blockIdx.x * 256 + threadIdx.x;
+    if (!buf || q >= (unsigned)nl * col.d * row.d) return;
+    const unsigned r = fdiv(q, row), ll = fdiv(r, col);
+    const int i = (int)(q - r * row.d), k = (int)(r - ll * col.d), l = l0 + (int)ll;
     const long long o = (long long)l * g.dstride + g.off(i, j, k);
+    buf += (long long)l0 * col.d * row.d;
     if (UNPACK) {
         f[o] = buf[q];
     } else {

@@ -163,19 +163,25 @@ class SlabTile:
 
 def step_local(tiles: list[SlabTile], n: int = 1):
     """n steps of all tiles of a domain held in one process (one device): each
-    tile steps, then the planes move between the tiles' buffers."""
+    tile steps and packs its planes into its neighbours' receive buffers, then
+    every tile unpacks its own."""
     cur = torch.cuda.current_stream()
+    streams = {t.lbm.stream.cuda_stream: t.lbm.stream for t in tiles}
+    alone = list(streams) == [cur.cuda_stream]     # one stream for all: already in order
+
+    def join():
+        if not alone:
+            for s in streams.values():
+                cur.wait_stream(s)
+            for s in streams.values():
+                s.wait_stream(cur)
+
     for _ in range(n):
+        join()                                     # the neighbours are done with what a pack overwrites
         for t in tiles:
             t.lbm.step(1)
-            t.pack()
+            t.lbm.halo_pack_j(tiles[t.south].recv[1] if t.south is not None else None,
+                              tiles[t.north].recv[0] if t.north is not None else None)
+        join()
         for t in tiles:
-            cur.wait_stream(t.lbm.stream)
-        for t in tiles:
-            if t.south is not None:
-                t.recv[0].copy_(tiles[t.south].send[1])
-            if t.north is not None:
-                t.recv[1].copy_(tiles[t.north].send[0])
-        for t in tiles:
-            t.lbm.stream.wait_stream(cur)
             t.unpack()
