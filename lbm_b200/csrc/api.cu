@@ -440,6 +440,19 @@ bool periodic_box(const lbm_ctx* c) {
     return c->p.ibnd == 0 && c->p.jbnd == 0 && c->p.kbnd == 0 && ghost_cells(c->sg) < (1LL << 31) - 128;
 }
 
+PullOffsets pull_offsets(const lbm_ctx* c) {
+    PullOffsets off;
+    memset(&off, 0, sizeof(off));
+    const SoaGrid& g = c->sg;
+    const long long plane = (long long)g.pitch * (g.ny + 2), elem = (long long)c->elem;
+    for (int l = 0; l < c->p.nl; ++l) {
+        const long long d = lat_cx(l) + (long long)lat_cy(l) * g.pitch + (long long)lat_cz(l) * plane;
+        off.poffb[l] = ((long long)l * g.dstride - d) * elem;
+        off.soffb[l] = (long long)l * g.dstride * elem;
+    }
+    return off;
+}
+
 StepArgs step_args(lbm_ctx* c) {
     StepArgs a;
     memset(&a, 0, sizeof(a));
@@ -475,17 +488,12 @@ StepArgs step_args(lbm_ctx* c) {
     a.full_sector = (c->p.nx % (32 / (int)c->elem)) == 0;
     a.xg_dst = c->d_xg[1 - c->cur];
     a.force = c->force;
-    {
-        const SoaGrid& g = c->sg;
-        const long long plane = (long long)g.pitch * (g.ny + 2);
-        for (int l = 0; l < c->p.nl; ++l) {
-            const long long d = lat_cx(l) + (long long)lat_cy(l) * g.pitch + (long long)lat_cz(l) * plane;
-            const long long po = (long long)l * g.dstride - d, so = (long long)l * g.dstride;
-            a.poff[l] = (int)po;   // read only when the state fits 32-bit offsets (idx32)
-            a.soff[l] = (int)so;
-            a.poffb[l] = po * (long long)c->elem;
-            a.soffb[l] = so * (long long)c->elem;
-        }
+    const PullOffsets off = pull_offsets(c);
+    for (int l = 0; l < c->p.nl; ++l) {
+        a.poffb[l] = off.poffb[l];
+        a.soffb[l] = off.soffb[l];
+        a.poff[l] = (int)(off.poffb[l] / (long long)c->elem);   // read only when the state fits 32-bit offsets (idx32)
+        a.soff[l] = (int)(off.soffb[l] / (long long)c->elem);
     }
     return a;
 }
@@ -704,8 +712,8 @@ template <int Q, typename S>
 void launch_export(lbm_ctx* c, float* f1, float* f2, int b) {
     const SoaGrid& g = c->sg;
     dim3 grd((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2);
-    k_export<Q, S, true><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], (const S*)c->buf[1 - b], f1, f2, g,
-                                                    wrap_rows(c), xg_of<S>(c, 1 - b), xg_of<S>(c, b));
+    launch_pdl(k_export<Q, S, true>, grd, dim3(128), c->stream, (const S*)c->buf[b], (const S*)c->buf[1 - b], f1, f2, g,
+               wrap_rows(c), xg_of<S>(c, 1 - b), xg_of<S>(c, b), pull_offsets(c));
     c->launches++;
 }
 // buffer b of an imported state as it is
@@ -714,15 +722,16 @@ void launch_export_stored(lbm_ctx* c, float* f, int b) {
     const SoaGrid& g = c->sg;
     dim3 grd((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2);
     k_export<Q, S, false><<<grd, 128, 0, c->stream>>>((const S*)c->buf[b], nullptr, f, nullptr, g, wrap_rows(c),
-                                                     xg_of<S>(c, b), nullptr);
+                                                     xg_of<S>(c, b), nullptr, pull_offsets(c));
     c->launches++;
 }
 template <int Q, typename S>
 void launch_macro(lbm_ctx* c, float* rho, float* u, float* v, float* w) {
     const SoaGrid& g = c->sg;
-    k_macro<Q, S><<<dim3((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2), 128, 0, c->stream>>>(
-        (const S*)c->buf[c->cur], (const S*)c->buf[1 - c->cur], rho, u, v, w, g, wrap_rows(c),
-        xg_of<S>(c, 1 - c->cur));
+    const int hp = (g.nx + 1) / 2, t = std::min(128, pair_width<Q, S>(hp));
+    launch_pdl(k_macro<Q, S>, dim3((unsigned)((hp + t - 1) / t), g.ny + 2, g.nz + 2), dim3(t), c->stream,
+               (const S*)c->buf[c->cur], (const S*)c->buf[1 - c->cur], rho, u, v, w, g, wrap_rows(c),
+               xg_of<S>(c, 1 - c->cur), pull_offsets(c));
     c->launches++;
 }
 
@@ -1480,9 +1489,9 @@ static void halo_planes(lbm_ctx* c, void* lo, void* hi, int jlo, int jhi, bool u
         using T = decltype(t);
         const dim3 grd((unsigned)((nl * per + 255) / 256), 2);
         if (unpack)
-            k_halo_planes<T, true><<<grd, 256, 0, c->stream>>>((T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
+            launch_pdl(k_halo_planes<T, true>, grd, dim3(256), c->stream, (T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
         else
-            k_halo_planes<T, false><<<grd, 256, 0, c->stream>>>((T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
+            launch_pdl(k_halo_planes<T, false>, grd, dim3(256), c->stream, (T*)lo, (T*)hi, (T*)f, c->sg, jlo, jhi, Q, (const T*)xg, row, col, l0, nl);
         c->launches++;
     };
     for (int l0 = 0; l0 < Q; l0 += most) {

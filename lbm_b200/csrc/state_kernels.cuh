@@ -527,6 +527,7 @@ inline long long fold_ghost_cells(const SoaGrid& g) {
 template <typename T, bool UNPACK>
 __global__ void __launch_bounds__(256) k_halo_planes(T* blo, T* bhi, T* f, SoaGrid g, int jlo, int jhi, int Q,
                                                      const T* __restrict__ xg, FastDiv row, FastDiv col, int l0, int nl) {
+    pdl_enter();
     T* buf = blockIdx.y ? bhi : blo;
     const int j = blockIdx.y ? jhi : jlo;
     const unsigned q = blockIdx.x * 256 + threadIdx.x;
@@ -807,6 +808,13 @@ struct PullMacro<Q, S, Q> {
     static __device__ __forceinline__ void run(float (&)[Q], const S*, const SoaGrid&, long long, int, bool) {}
 };
 
+// Byte offsets of direction l from a cell: its pull source and its own entry (one
+// constant operand per address, where computing them takes a dozen instructions
+// a load and binds the read-back kernels).
+struct PullOffsets {
+    long long poffb[27], soffb[27];
+};
+
 // A chunk of n cells (one thread each, row (j,k), first cell i0) of the
 // reference layout from a tile staged at sm[t Q + l + phase]: whole 16-byte
 // words where the chunk covers them.
@@ -837,8 +845,10 @@ __device__ __forceinline__ void export_put(const float* sm, float* out, int n) {
 template <int Q, typename S, bool PULL>
 __global__ void __launch_bounds__(128) k_export(const S* __restrict__ src, const S* __restrict__ ghost,
                                                 float* __restrict__ ref1, float* __restrict__ ref2, SoaGrid g, int wrap,
-                                                const S* __restrict__ xg1, const S* __restrict__ xg2) {
+                                                const S* __restrict__ xg1, const S* __restrict__ xg2,
+                                                const PullOffsets off) {
     __shared__ __align__(16) float sm[128 * Q + 4];
+    pdl_enter();
     const int i0 = blockIdx.x * 128;
     const int j = blockIdx.y, k = blockIdx.z;
     const int n = min(128, g.nx + 2 - i0);
@@ -851,11 +861,14 @@ __global__ void __launch_bounds__(128) k_export(const S* __restrict__ src, const
     const long long xl = (long long)g.ny * g.nz, o = g.off(i, jw, k);
     float v[Q];
     auto cell_of = [&](const S* s, const S* xg) {
-        const bool x = xg && xghost;
-        const S* p = x ? xg + xo : s + o;
-        const long long step = x ? xl : g.dstride;
+        if (xg && xghost) {
 #pragma unroll
-        for (int l = 0; l < Q; ++l) v[l] = Store<S>::to_f(p[l * step]);
+            for (int l = 0; l < Q; ++l) v[l] = Store<S>::to_f(xg[xo + l * xl]);
+        } else {
+            const char* p = reinterpret_cast<const char*>(s + o);
+#pragma unroll
+            for (int l = 0; l < Q; ++l) v[l] = Store<S>::to_f(*reinterpret_cast<const S*>(p + off.soffb[l]));
+        }
     };
     auto stage = [&](float* out) {
         float* p = sm + phase_of(out) + t * Q;
@@ -868,10 +881,19 @@ __global__ void __launch_bounds__(128) k_export(const S* __restrict__ src, const
     };
     if (PULL) {
         if (t < n) {
-            if (i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz)
-                PullMacro<Q, S, 0>::run(v, src, g, g.off(i, j, k), j, wrap != 0);
-            else
+            if (i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz) {
+                // a source row 0 or ny+1 is row ny or 1 with wrap
+                const S* p0 = src + g.off(i, j, k);
+                const S* pp = (wrap && j == 1) ? p0 + (long long)g.ny * g.pitch : p0;
+                const S* pm = (wrap && j == g.ny) ? p0 - (long long)g.ny * g.pitch : p0;
+#pragma unroll
+                for (int l = 0; l < Q; ++l) {
+                    const S* p = lat_cy(l) > 0 ? pp : (lat_cy(l) < 0 ? pm : p0);
+                    v[l] = Store<S>::to_f(*reinterpret_cast<const S*>(reinterpret_cast<const char*>(p) + off.poffb[l]));
+                }
+            } else {
                 cell_of(ghost, xg1);
+            }
         }
         stage(ref1 + base);
         if (t < n) cell_of(src, xg2);
@@ -881,37 +903,6 @@ __global__ void __launch_bounds__(128) k_export(const S* __restrict__ src, const
         if (t < n) cell_of(src, xg1);
         stage(ref1 + base);
     }
-}
-
-// macrovars of the reference's f1 without materialising it: interior cells
-// from the pulled values of `src`, ghost cells from `ghost` itself.
-template <int Q, typename S>
-__global__ void __launch_bounds__(128) k_macro(const S* __restrict__ src, const S* __restrict__ ghost, float* rho,
-                                               float* u, float* v, float* w, SoaGrid g, int wrap,
-                                               const S* __restrict__ xg) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i > g.nx + 1) return;
-    const bool interior = i >= 1 && i <= g.nx && j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
-    float fp[Q];
-    if (interior) {
-        PullMacro<Q, S, 0>::run(fp, src, g, g.off(i, j, k), j, wrap != 0);
-    } else {
-        const int jw = wrap ? wrapj(j, g.ny) : j;
-        const long long o = g.off(i, jw, k);
-        const bool fromxg = xg && (i == 0 || i == g.nx + 1) && jw >= 1 && jw <= g.ny && k >= 1 && k <= g.nz;
-#pragma unroll
-        for (int l = 0; l < Q; ++l)
-            fp[l] = Store<S>::to_f(fromxg ? xg[xg_index(g, Q, i == 0 ? 0 : 1, l, jw, k)] : ghost[(long long)l * g.dstride + o]);
-    }
-    const Moments m = moments<Q>(fp);
-    const float r = 1.0f + m.s0;
-    const float inv = 1.0f / r;
-    const long long c = (long long)i + (long long)(g.nx + 2) * ((long long)j + (long long)(g.ny + 2) * k);
-    rho[c] = r;
-    u[c] = m.jx * inv;
-    v[c] = m.jy * inv;
-    w[c] = m.jz * inv;
 }
 
 }  // namespace lbm
