@@ -48,12 +48,17 @@ class ProbeProblem:
     # ---- forward ----------------------------------------------------------------------
     def _macro(self, f):
         L = self.lbm
-        R = [L.empty_s(self.dtype) for _ in range(4)]
+        R = self._fields()
         L.macrovars(*R, f)
         return R
 
-    def _step(self, A, B, R, uvel):
-        """one step in place of main.F90's order; returns the new (f1, f2)"""
+    def _fields(self):
+        """rho, u, v, w for macrovars, which writes every cell"""
+        return [torch.empty(self.p.sshape, dtype=self.dtype, device="cuda") for _ in range(4)]
+
+    def _step(self, A, B, R, uvel, out=None):
+        """one step in place of main.F90's order; returns the new (f1, f2).  out: where
+        the new rho, u, v, w go (default: in place of R)"""
         L = self.lbm
         L.postcoll(A, self.tau, *R)
         if self.blanking is not None:
@@ -61,7 +66,7 @@ class ProbeProblem:
         L.boundarycond(A, B, uvel)
         L.drift(B, A)
         A, B = B, A
-        L.macrovars(*R, A)
+        L.macrovars(*(R if out is None else out), A)
         return A, B
 
     def probe_u(self, R):
@@ -97,8 +102,9 @@ class ProbeProblem:
             R = self._macro(A)
             states = []                       # (A_n, R_n) of the segment
             for n in range(s, e):
-                states.append((A.clone(), [t.clone() for t in R]))
-                A, B = self._step(A, B, R, self.uvel)
+                states.append((A.clone(), R))
+                R = self._fields()
+                A, B = self._step(A, B, states[-1][1], self.uvel, out=R)
             R_next = R
             for n in range(e - 1, s - 1, -1):
                 A_n, R_n = states[n - s]

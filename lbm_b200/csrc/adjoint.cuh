@@ -227,47 +227,94 @@ __device__ __forceinline__ void collide_adj(const float (&fp)[Q], const float (&
 // rhoh, uh, vh, wh are incremented.  f, rho, u, v, w, tau, abl: postcoll's inputs.
 // blank (may be null): the adjoint of a solids call that followed postcoll is
 // applied first (a swap of opposite directions at blanked cells).
+// Tiles as k_ref_postcoll's (ref_kernels.cuh): the next tile's two arrays and
+// scalars arrive while this one is worked on (a block that loaded, computed and
+// stored in turn: 54 us for D3Q19 128x64x64, 2.5 TB/s).
 template <int Q>
-__global__ void __launch_bounds__(128) k_ref_postcoll_adj(float* fh, const float* f, const float* rho, const float* u,
-                                                          const float* v, const float* w, const float* tau,
-                                                          const float* abl, float* rhoh, float* uh, float* vh,
-                                                          float* wh, const int32_t* blank, RefGrid g, CollideParams cp) {
-    __shared__ float sf[128 * Q];
-    __shared__ float sg[128 * Q];
-    const int i0 = blockIdx.x * 128 + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
-    const int n = min(128, g.nx + 1 - i0);
-    const int t = threadIdx.x;
-    if (n <= 0) return;
-    tile_load<Q>(sf, f, g.cell(i0, j, k), n);
-    tile_load<Q>(sg, fh, g.cell(i0, j, k), n);
-    __syncthreads();
-    if (t < n) {
-        const long long c = g.cell(i0 + t, j, k);
-        float fp[Q], gh[Q], out[Q];
-#pragma unroll
-        for (int l = 0; l < Q; ++l) {
-            fp[l] = sf[t * Q + l] - lat_w<Q>(l);
-            gh[l] = sg[t * Q + l];
+struct PostcollAdjTile {
+    static constexpr int SC = 9;                                    // rho, u, v, w, tau and the four adjoints
+    static constexpr int STAGE = 2 * CellTile<Q, float>::BUF + SC * CELL_T;
+    static constexpr size_t SMEM = 2 * STAGE * sizeof(float);
+    static constexpr int BLOCKS = Q == 27 ? 3 : 4;
+};
+template <int Q>
+__global__ void __launch_bounds__(CELL_T, PostcollAdjTile<Q>::BLOCKS)
+    k_ref_postcoll_adj(float* fh, const float* f, const float* rho, const float* u, const float* v, const float* w,
+                       const float* tau, const float* abl, float* rhoh, float* uh, float* vh, float* wh,
+                       const int32_t* blank, RefGrid g, CollideParams cp, unsigned tp, unsigned ntiles) {
+    using P = PostcollAdjTile<Q>;
+    constexpr int BUF = CellTile<Q, float>::BUF;
+    extern __shared__ __align__(16) unsigned char raw[];
+    __shared__ unsigned cells[CELL_T / 32];
+    float* sm = reinterpret_cast<float*>(raw);
+    const int tid = threadIdx.x;
+    auto fetch = [&](unsigned t, int b) {
+        const TileAt a = tile_at<false>(g, t, tp);
+        float* s = sm + b * P::STAGE;
+        tile_fetch<Q>(s, f, a.c0, a.n);
+        tile_fetch<Q>(s + BUF, fh, a.c0, a.n);
+        if (tid < a.n) {
+            s += 2 * BUF + tid;
+            const long long c = a.c0 + tid;
+            cp_async_elem(s, rho + c);
+            cp_async_elem(s + CELL_T, u + c);
+            cp_async_elem(s + 2 * CELL_T, v + c);
+            cp_async_elem(s + 3 * CELL_T, w + c);
+            cp_async_elem(s + 4 * CELL_T, tau + c);
+            cp_async_elem(s + 5 * CELL_T, rhoh + c);
+            cp_async_elem(s + 6 * CELL_T, uh + c);
+            cp_async_elem(s + 7 * CELL_T, vh + c);
+            cp_async_elem(s + 8 * CELL_T, wh + c);
         }
-        if (blank && blank[c] != 0) {
+    };
+    fetch(blockIdx.x, 0);
+    cp_async_commit();
+    int b = 0;
+    for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
+        if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
+        cp_async_commit();
+        const TileAt a = tile_at<false>(g, t, tp);
+        const unsigned i = (a.q0 + tid) % (unsigned)(g.nx + 2);
+        const bool inner = tid < a.n && i >= 1 && i <= (unsigned)g.nx;
+        const unsigned mask = __ballot_sync(0xffffffffu, inner);
+        if ((tid & 31) == 0) cells[tid >> 5] = mask;
+        const long long c = a.c0 + tid;
+        const bool solid = inner && blank && blank[c] != 0;
+        cp_async_wait<1>();
+        __syncthreads();
+        float* tile = sm + b * P::STAGE;
+        if (inner) {
+            const float* sf = tile + phase_of(f + a.c0 * Q) + tid * Q;
+            float* sg = tile + BUF + phase_of(fh + a.c0 * Q) + tid * Q;
+            const float* sc = tile + 2 * BUF + tid;
+            float fp[Q], gh[Q], out[Q];
 #pragma unroll
-            for (int l = 1; l + 1 < Q; l += 2) {
-                const float x = gh[l];
-                gh[l] = gh[l + 1];
-                gh[l + 1] = x;
+            for (int l = 0; l < Q; ++l) {
+                fp[l] = sf[l] - lat_w<Q>(l);
+                gh[l] = sg[l];
             }
-        }
-        float rr = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-        collide_adj<Q>(fp, gh, rho[c], u[c], v[c], w[c], cp, abl ? abl[k - 1] : 0.0f, tau[c], out, rr, ux, uy, uz);
-        rhoh[c] += rr;
-        uh[c] += ux;
-        vh[c] += uy;
-        wh[c] += uz;
+            if (solid) {
 #pragma unroll
-        for (int l = 0; l < Q; ++l) sg[t * Q + l] = out[l];
+                for (int l = 1; l + 1 < Q; l += 2) {
+                    const float x = gh[l];
+                    gh[l] = gh[l + 1];
+                    gh[l + 1] = x;
+                }
+            }
+            float rr = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+            collide_adj<Q>(fp, gh, sc[0], sc[CELL_T], sc[2 * CELL_T], sc[3 * CELL_T], cp, abl ? abl[a.k - 1] : 0.0f,
+                           sc[4 * CELL_T], out, rr, ux, uy, uz);
+            rhoh[c] = sc[5 * CELL_T] + rr;
+            uh[c] = sc[6 * CELL_T] + ux;
+            vh[c] = sc[7 * CELL_T] + uy;
+            wh[c] = sc[8 * CELL_T] + uz;
+#pragma unroll
+            for (int l = 0; l < Q; ++l) sg[l] = out[l];
+        }
+        const bool whole = __syncthreads_and(inner);
+        tile_put<Q>(tile + BUF, fh, a.c0, a.n, cells, whole);
+        __syncthreads();
     }
-    __syncthreads();
-    tile_store<Q>(sg, fh, g.cell(i0, j, k), n);
 }
 
 // macrovars adjoint over the ghost-inclusive grid: fh += d(rho, u, v, w)/df^T (rhoh, uh, vh, wh)
@@ -313,61 +360,10 @@ __global__ void __launch_bounds__(128) k_ref_macrovars_adj(float* fh, const floa
     tile_store<Q>(sg, fh, g.cell(i0, j, k), n);
 }
 
-// Per-direction tables of the drift adjoints, in shared memory: a constant read
-// indexed by l would serialise over the different directions of a warp.
-template <int Q>
-struct DriftTab {
-    int cx[Q], cy[Q], cz[Q];
-    long long d[Q];   // cell distance cx + (nx+2) cy + (nx+2)(ny+2) cz
-};
-template <int Q>
-__device__ __forceinline__ void drift_tab(DriftTab<Q>& t, const RefGrid& g) {
-    if (threadIdx.x < Q) {
-        const int l = threadIdx.x;
-        t.cx[l] = lat_cx(l);
-        t.cy[l] = lat_cy(l);
-        t.cz[l] = lat_cz(l);
-        t.d[l] = lat_cx(l) + (long long)lat_cy(l) * (g.nx + 2) + (long long)lat_cz(l) * (g.nx + 2) * (g.ny + 2);
-    }
-    __syncthreads();
-}
-#define DRIFT_ADJ_ILP 4
-
-// drift adjoint: fh_in(l, y) += fh_out(l, y + c_l) for y + c_l interior (the
-// transpose of the pull).  One block per row (j,k) of the ghost-inclusive grid,
-// looping over its (nx+2)*Q entries, DRIFT_ADJ_ILP loads in flight per thread.
-template <int Q>
-__global__ void __launch_bounds__(256) k_ref_drift_adj(float* __restrict__ fh_in, const float* __restrict__ fh_out,
-                                                       RefGrid g) {
-    __shared__ DriftTab<Q> t;
-    drift_tab<Q>(t, g);
-    const int j = blockIdx.x, k = blockIdx.y;
-    const long long c0 = g.cell(0, j, k);
-    const int n = Q * (g.nx + 2);
-    for (int e0 = threadIdx.x; e0 < n; e0 += blockDim.x * DRIFT_ADJ_ILP) {
-        float val[DRIFT_ADJ_ILP];
-        bool ok[DRIFT_ADJ_ILP];
-#pragma unroll
-        for (int u = 0; u < DRIFT_ADJ_ILP; ++u) {
-            const int e = e0 + u * blockDim.x;
-            ok[u] = false;
-            if (e >= n) continue;
-            const int l = e % Q, i = e / Q;
-            const int ti = i + t.cx[l], tj = j + t.cy[l], tk = k + t.cz[l];
-            if (ti < 1 || ti > g.nx || tj < 1 || tj > g.ny || tk < 1 || tk > g.nz) continue;
-            ok[u] = true;
-            val[u] = fh_in[c0 * Q + e] + fh_out[(c0 + i + t.d[l]) * Q + l];
-        }
-#pragma unroll
-        for (int u = 0; u < DRIFT_ADJ_ILP; ++u)
-            if (ok[u]) fh_in[c0 * Q + e0 + u * blockDim.x] = val[u];
-    }
-}
-
 // The macrovars adjoint at a cell x, as four terms: with a = (uh, vh, wh) / rho,
 // d(rho, u)/df_l^T (rhoh, uh, vh, wh) = (rhoh - a.u) + a.c_l.  One thread per
-// interior cell; T is [4][cells of the ghost-inclusive grid].
-__global__ void __launch_bounds__(256) k_ref_macro_adj_terms(float* __restrict__ T, const float* __restrict__ rhoh,
+// interior cell; T has the ghost-inclusive grid's cells.
+__global__ void __launch_bounds__(256) k_ref_macro_adj_terms(float4* __restrict__ T, const float* __restrict__ rhoh,
                                                              const float* __restrict__ uh, const float* __restrict__ vh,
                                                              const float* __restrict__ wh, const float* __restrict__ rho,
                                                              const float* __restrict__ u, const float* __restrict__ v,
@@ -375,49 +371,132 @@ __global__ void __launch_bounds__(256) k_ref_macro_adj_terms(float* __restrict__
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y + 1, k = blockIdx.z + 1;
     if (i > g.nx) return;
-    const long long x = g.cell(i, j, k), n = g.ncell();
+    const long long x = g.cell(i, j, k);
     const float inv = 1.0f / rho[x];
     const float ax = uh[x] * inv, ay = vh[x] * inv, az = wh[x] * inv;
-    T[x] = rhoh[x] - (ax * u[x] + ay * v[x] + az * w[x]);
-    T[n + x] = ax;
-    T[2 * n + x] = ay;
-    T[3 * n + x] = az;
+    T[x] = make_float4(rhoh[x] - (ax * u[x] + ay * v[x] + az * w[x]), ax, ay, az);
 }
 
-// drift adjoint preceded by the adjoint of the macrovars call that followed the
-// drift: fh_in(l, y) += fh_out(l, x) + d(rho, u)(x)/df_l^T (rhoh, uh, vh, wh)(x)
+// drift adjoint: fh_in(l, y) += fh_out(l, y + c_l) for y + c_l interior (the transpose of
+// the pull).  MACRO: preceded by the adjoint of the macrovars call that followed
+// the drift, fh_in(l, y) += fh_out(l, x) + d(rho, u)(x)/df_l^T (rhoh, uh, vh, wh)(x)
 // for x = y + c_l interior, where rho(x), u(x) are the macrovars outputs and T
-// holds the four terms of k_ref_macro_adj_terms.  The macrovars adjoints are
-// taken at interior cells only.  Layout and loop as k_ref_drift_adj.
-template <int Q>
-__global__ void __launch_bounds__(256) k_ref_macro_drift_adj(float* __restrict__ fh_in,
-                                                             const float* __restrict__ fh_out,
-                                                             const float* __restrict__ T, RefGrid g) {
-    __shared__ DriftTab<Q> t;
-    drift_tab<Q>(t, g);
-    const int j = blockIdx.x, k = blockIdx.y;
-    const long long c0 = g.cell(0, j, k), nc = g.ncell();
-    const int n = Q * (g.nx + 2);
-    for (int e0 = threadIdx.x; e0 < n; e0 += blockDim.x * DRIFT_ADJ_ILP) {
-        float val[DRIFT_ADJ_ILP];
-        bool ok[DRIFT_ADJ_ILP];
+// holds the four terms of k_ref_macro_adj_terms (interior cells).
+// The ring of k_ref_drift (ref_kernels.cuh) over the ghost-inclusive grid, read
+// at y + c_l; with MACRO a plane also holds its cells' four terms.  (Gathered
+// from global memory, one sector per element: 53 us for D3Q19 128x64x64.)  The
+// words at a row's ends bring neighbours along; a word that reaches past the
+// array holds nothing that is used, since the ghosts around it are not.
+template <int Q, bool MACRO>
+struct DriftAdjTile {
+    using D = DriftTile<Q, float>;
+    static constexpr int TC = D::NI + 2;                            // cells of a row
+    static constexpr int TPS = MACRO ? 4 * (D::TJ + 2) * TC : 0;    // terms of a plane
+    static constexpr int SLOTS = MACRO ? D::SLOTS - 1 : D::SLOTS;   // the terms take the room of a plane
+    static constexpr int AHEAD = SLOTS - 3;
+    static constexpr size_t SMEM = (size_t)SLOTS * (D::PS + TPS) * sizeof(float);
+    static_assert(D::BLOCKS * (SMEM + 1024) <= 228 * 1024, "the blocks fit an SM");
+};
+template <int Q, bool MACRO>
+__global__ void __launch_bounds__(DriftTile<Q, float>::T, DriftTile<Q, float>::BLOCKS)
+    k_ref_drift_adj(float* __restrict__ fh_in, const float* __restrict__ fh_out, const float4* __restrict__ T, RefGrid g,
+                    DriftShape d) {
+    using D = DriftTile<Q, float>;
+    using A = DriftAdjTile<Q, MACRO>;
+    constexpr int V = D::V, TJ = D::TJ, M = D::NI / D::LANES;
+    constexpr int LOADS = ((TJ + 2) * D::WORDS + D::T - 1) / D::T;   // words a thread copies per plane
+    static_assert((TJ + 2) * A::TC <= D::T, "a thread copies at most one cell's terms per plane");
+    extern __shared__ __align__(16) unsigned char raw[];
+    float* sm = reinterpret_cast<float*>(raw);
+    float4* st = reinterpret_cast<float4*>(sm + A::SLOTS * D::PS);
+    const int tid = threadIdx.x;
+    // y: cells i0 .. i0 + ni - 1 of the rows j0 .., planes k0 .., of the grid with ghosts
+    const int w = g.nx + 2, nch = (w + d.ni - 1) / d.ni, jt = blockIdx.x / nch;
+    const int i0 = (blockIdx.x - jt * nch) * d.ni, j0 = jt * TJ, k0 = blockIdx.y * d.ks;
+    const int ni = min(d.ni, w - i0), nj = min(TJ, g.ny + 2 - j0), k1 = min(k0 + d.ks, g.nz + 2);
+    if (ni <= 0 || nj <= 0 || k0 >= k1) return;
+    const int np = k1 - k0, len = (ni + 2) * Q;
+    const long long rowg = (long long)w * Q, planec = (long long)w * (g.ny + 2), planeg = planec * Q, nc = g.ncell();
+    const long long cell0 = (long long)(i0 - 1) + (long long)w * (j0 - 1) + planec * (k0 - 1);   // may lie before the array
+    const int ph0 = (int)(((phase_of(fh_out) + cell0 * Q) % V + V) % V);
+    int lr[LOADS], lw[LOADS];
 #pragma unroll
-        for (int q = 0; q < DRIFT_ADJ_ILP; ++q) {
-            const int e = e0 + q * blockDim.x;
-            ok[q] = false;
-            if (e >= n) continue;
-            const int l = e % Q, i = e / Q;
-            const int cx = t.cx[l], cy = t.cy[l], cz = t.cz[l];
-            const int ti = i + cx, tj = j + cy, tk = k + cz;
-            if (ti < 1 || ti > g.nx || tj < 1 || tj > g.ny || tk < 1 || tk > g.nz) continue;
-            ok[q] = true;
-            const long long x = c0 + i + t.d[l];
-            const float m = T[x] + (T[nc + x] * (float)cx + T[2 * nc + x] * (float)cy + T[3 * nc + x] * (float)cz);
-            val[q] = fh_in[c0 * Q + e] + (fh_out[x * Q + l] + m);
+    for (int q = 0; q < LOADS; ++q) {
+        const int e = tid + q * D::T;
+        lr[q] = e / D::WORDS;
+        lw[q] = e - lr[q] * D::WORDS;
+    }
+    const int tr = tid / A::TC, tcell = tid - tr * A::TC;
+    // the interior rows of plane p (k = k0 - 1 + p), if it is one, into ring slot `slot`
+    auto load_plane = [&](int p, int slot) {
+        if (k0 - 1 + p < 1 || k0 - 1 + p > g.nz) return;
+        const long long eo = cell0 * Q + p * planeg;
+        const int at = slot * D::PS + (int)((ph0 + p * planeg) & (V - 1));
+#pragma unroll
+        for (int q = 0; q < LOADS; ++q) {
+            const int j = j0 - 1 + lr[q];
+            if (lr[q] >= nj + 2) break;
+            const int o = at + lr[q] * d.rs, ph = o % V;
+            const long long e = eo + lr[q] * rowg - ph + lw[q] * V;
+            if (j >= 1 && j <= g.ny && lw[q] * V < ph + len && e >= 0 && e + V <= nc * Q)
+                cp_async16(sm + (o - ph) + lw[q] * V, fh_out + e);
         }
+        if (MACRO) {
+            const int j = j0 - 1 + tr;
+            const long long c = cell0 + p * planec + (long long)tr * w + tcell;
+            if (tr < nj + 2 && j >= 1 && j <= g.ny && tcell < ni + 2 && c >= 0 && c < nc)
+                cp_async16(st + slot * (A::TPS / 4) + tid, T + c);
+        }
+    };
 #pragma unroll
-        for (int q = 0; q < DRIFT_ADJ_ILP; ++q)
-            if (ok[q]) fh_in[c0 * Q + e0 + q * blockDim.x] = val[q];
+    for (int p = 0; p < 2 + A::AHEAD; ++p) {
+        if (p < np + 2) load_plane(p, p);
+        cp_async_commit();
+    }
+    const int l = tid % Q, lane = tid / Q;
+    const int cx = c_cx[l], cy = c_cy[l], cz = c_cz[l];
+    const float fx = (float)cx, fy = (float)cy, fz = (float)cz;
+    const int from = (1 + cy) * d.rs + (1 + cx) * Q + tid;
+    // the entries of this thread whose target cell and row are interior
+    unsigned on = 0;
+#pragma unroll
+    for (int r = 0; r < TJ; ++r)
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int c = lane + m * D::LANES, x = i0 + c + cx, y = j0 + r + cy;
+            if (c < ni && r < nj && x >= 1 && x <= g.nx && y >= 1 && y <= g.ny) on |= 1u << (r * M + m);
+        }
+    float* dst = fh_in + (cell0 + 1 + w + planec) * Q + tid;
+    int slot = 1, next = 2 + A::AHEAD;
+    for (int p = 0; p < np; ++p) {
+        const int kt = k0 + p + cz;
+        const unsigned now = (kt >= 1 && kt <= g.nz) ? on : 0u;
+        // this plane's entries, fetched while the ring's planes arrive
+        float v[TJ * M];
+#pragma unroll
+        for (int q = 0; q < TJ * M; ++q)
+            if (now >> q & 1u) v[q] = dst[(q / M) * rowg + (q % M) * D::T];
+        cp_async_wait<A::AHEAD - 1>();
+        __syncthreads();
+        if (p + 2 + A::AHEAD < np + 2) load_plane(p + 2 + A::AHEAD, next);
+        cp_async_commit();
+        int at = slot + cz;
+        at += at < 0 ? A::SLOTS : (at >= A::SLOTS ? -A::SLOTS : 0);
+        const float* s = sm + at * D::PS + (int)((ph0 + (p + 1 + cz) * planeg) & (V - 1)) + from;
+        const float4* t = st + at * (A::TPS / 4) + (1 + cy) * A::TC + 1 + cx + lane;
+#pragma unroll
+        for (int q = 0; q < TJ * M; ++q) {
+            if (!(now >> q & 1u)) continue;
+            float x = s[(q / M) * d.rs + (q % M) * D::T];
+            if (MACRO) {
+                const float4 h = t[(q / M) * A::TC + (q % M) * D::LANES];
+                x += h.x + (h.y * fx + h.z * fy + h.w * fz);
+            }
+            dst[(q / M) * rowg + (q % M) * D::T] = v[q] + x;
+        }
+        dst += planeg;
+        slot = slot + 1 == A::SLOTS ? 0 : slot + 1;
+        next = next + 1 == A::SLOTS ? 0 : next + 1;
     }
 }
 
@@ -526,6 +605,42 @@ __global__ void k_periodic_adj(Acc a, int axis, int nl, int skipj) {
         *sn = wn + v0;
         *s1 = w1 + v1;
     }
+}
+
+// reverse of k_ref_periodic (ref_kernels.cuh; same threads): the ghost planes of the
+// axis pass their adjoints to the planes they were copied from.  kfaces: of
+// axis 1 only the planes k = 1 and nz (grid y = 2), the only ones whose j ghosts
+// hold anything after the second round's reverse when nothing but closed k faces
+// read them in between.
+__global__ void __launch_bounds__(256) k_ref_periodic_adj(float* __restrict__ f, RefGrid g, int axis, int kfaces) {
+    const long long row = (long long)(g.nx + 2) * g.nl, plane = row * (g.ny + 2);
+    const long long e = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int k = kfaces ? (blockIdx.y ? g.nz : 1) : blockIdx.y;
+    long long at, step;
+    int n;
+    if (axis == 0) {
+        const long long j = e / g.nl;
+        if (j > g.ny + 1) return;
+        at = j * row + (e - j * g.nl) + k * plane;
+        step = g.nl;
+        n = g.nx;
+    } else if (axis == 1) {
+        if (e >= row) return;
+        at = e + k * plane;
+        step = row;
+        n = g.ny;
+    } else {
+        if (e >= plane) return;
+        at = e;
+        step = plane;
+        n = g.nz;
+    }
+    float* p = f + at;
+    const float v0 = p[0], v1 = p[(n + 1) * step], wn = p[n * step], w1 = p[step];
+    p[0] = 0.0f;
+    p[(n + 1) * step] = 0.0f;
+    p[n * step] = wn + v0;
+    p[step] = w1 + v1;
 }
 
 // reverse of k_closed (same grid): per pair, f1(m,G) = f2(l,G) and

@@ -15,7 +15,15 @@ template <int Q, typename AdjA>
 int run_bc_adj(lbm_ctx* c, AdjA a1, AdjA a2, float* uvelh, bool wrap = false) {
     const int nx = c->p.nx, ny = c->p.ny, nz = c->p.nz, nl = c->p.nl;
     cudaStream_t s = c->stream;
-    auto periodic = [&](int axis) {
+    auto periodic = [&](int axis, bool kfaces = false) {
+        if constexpr (std::is_same<AdjA, AdjAcc>::value) {
+            const long long row = (long long)(nx + 2) * Q;
+            const long long n = axis == 0 ? (long long)(ny + 2) * Q : axis == 1 ? row : row * (ny + 2);
+            k_ref_periodic_adj<<<dim3((unsigned)((n + 255) / 256), axis == 2 ? 1 : kfaces ? 2 : nz + 2), 256, 0, s>>>(
+                a1.f, c->rg, axis, kfaces ? 1 : 0);
+            c->launches++;
+            return;
+        }
         dim3 grd;
         if (axis == 0) grd = dim3((ny + 2 + 127) / 128, nz + 2, nl);
         else if (axis == 1) grd = dim3((nx + 2 + 127) / 128, nz + 2, nl);
@@ -47,9 +55,31 @@ int run_bc_adj(lbm_ctx* c, AdjA a1, AdjA a2, float* uvelh, bool wrap = false) {
         k_closed_adj<AdjA><<<dim3((na + 127) / 128, nb, 2), 128, 0, s>>>(a1, a2, a, c->face[a][0], c->face[a][1]);
         c->launches++;
     }
+    // the first round's copies: the second round's reverse has emptied every ghost; since
+    // then only the faces have added to j ghosts, the closed k faces in the planes 1 and nz
+    const bool kfaces = c->face_on[2] && !c->face_on[0] && codes[0] != 0;
     for (int a = 2; a >= 0; --a)
-        if (codes[a] == 0 && !(wrap && a == 1)) periodic(a);
+        if (codes[a] == 0 && !(wrap && a == 1)) periodic(a, a == 1 && kfaces);
     LBM_LAUNCHED(c, "boundarycond adjoint");
+    return LBM_OK;
+}
+
+// the drift adjoint over the ghost-inclusive grid, then the consumed interior cleared;
+// T: the macrovars adjoint's terms, or null
+template <int Q, bool MACRO>
+int drift_adj_launch(lbm_ctx* c, float* fhat_in, float* fhat_out, const float4* T) {
+    using D = DriftTile<Q, float>;
+    constexpr size_t smem = DriftAdjTile<Q, MACRO>::SMEM;
+    const RefGrid all{c->p.nx + 2, c->p.ny + 2, c->p.nz + 2, Q};     // its extents as the shape's
+    DriftShape d = drift_shape<Q, float>(all, c->nsm * D::BLOCKS);
+    d.rs = drift_row_stride<Q, float>(c->rg);
+    const dim3 grd((all.nx + d.ni - 1) / d.ni * ((all.ny + D::TJ - 1) / D::TJ), (all.nz + d.ks - 1) / d.ks);
+    LBM_TRY(cuda_check(c, cudaFuncSetAttribute(k_ref_drift_adj<Q, MACRO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem), "drift adjoint"));
+    k_ref_drift_adj<Q, MACRO><<<grd, D::T, smem, c->stream>>>(fhat_in, fhat_out, T, c->rg, d);
+    k_ref_zero_interior<<<dim3(c->p.ny, c->p.nz), 256, 0, c->stream>>>(fhat_out, c->rg);
+    c->launches += 2;
+    LBM_LAUNCHED(c, "drift adjoint");
     return LBM_OK;
 }
 
@@ -66,18 +96,16 @@ int lbm_postcoll_adj(lbm_ctx* c, float* fhat, const float* f, const float* tau, 
     if (!c->p.ivreman) NEED(c, tau);
     if (c->p.ihrr != 1)
         return fail(c, LBM_ERR_UNSUPPORTED, "postcoll_adj: the adjoint covers the regularized collision (ihrr = 1)");
-    dim3 grd((c->p.nx + 127) / 128, c->p.ny, c->p.nz);
     // with Vreman the forward computes tau itself; any array stands in for the unused input
     const float* t = tau ? tau : rho;
+    const unsigned tp = plane_tiles(c->rg), nt = tp * (unsigned)c->p.nz;
     if (c->p.nl == 27)
-        k_ref_postcoll_adj<27><<<grd, 128, 0, c->stream>>>(fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
-                                                           blanking, c->rg, c->cp);
-    else
-        k_ref_postcoll_adj<19><<<grd, 128, 0, c->stream>>>(fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
-                                                           blanking, c->rg, c->cp);
-    c->launches++;
-    LBM_LAUNCHED(c, "postcoll adjoint");
-    return LBM_OK;
+        return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<27>, PostcollAdjTile<27>::SMEM,
+                            PostcollAdjTile<27>::BLOCKS, nt, fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
+                            blanking, c->rg, c->cp, tp);
+    return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<19>, PostcollAdjTile<19>::SMEM,
+                        PostcollAdjTile<19>::BLOCKS, nt, fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
+                        blanking, c->rg, c->cp, tp);
 }
 
 int lbm_macrovars_adj(lbm_ctx* c, float* fhat, const float* rhohat, const float* uhat, const float* vhat,
@@ -96,13 +124,8 @@ int lbm_drift_adj(lbm_ctx* c, float* fhat_in, float* fhat_out) {
     if (!c) return LBM_ERR_ARG;
     NEED(c, fhat_in); NEED(c, fhat_out);
     if (fhat_in == fhat_out) return fail(c, LBM_ERR_ARG, "drift_adj: the two adjoint arrays must be distinct");
-    const dim3 grd(c->p.ny + 2, c->p.nz + 2);
-    if (c->p.nl == 27) k_ref_drift_adj<27><<<grd, 256, 0, c->stream>>>(fhat_in, fhat_out, c->rg);
-    else k_ref_drift_adj<19><<<grd, 256, 0, c->stream>>>(fhat_in, fhat_out, c->rg);
-    k_ref_zero_interior<<<dim3(c->p.ny, c->p.nz), 256, 0, c->stream>>>(fhat_out, c->rg);
-    c->launches += 2;
-    LBM_LAUNCHED(c, "drift adjoint");
-    return LBM_OK;
+    return c->p.nl == 27 ? drift_adj_launch<27, false>(c, fhat_in, fhat_out, nullptr)
+                         : drift_adj_launch<19, false>(c, fhat_in, fhat_out, nullptr);
 }
 
 int lbm_macrovars_drift_adj(lbm_ctx* c, float* fhat_in, float* fhat_out, const float* rhohat, const float* uhat,
@@ -112,19 +135,14 @@ int lbm_macrovars_drift_adj(lbm_ctx* c, float* fhat_in, float* fhat_out, const f
     NEED(c, fhat_in); NEED(c, fhat_out); NEED(c, rhohat); NEED(c, uhat); NEED(c, vhat); NEED(c, what);
     NEED(c, rho); NEED(c, u); NEED(c, v); NEED(c, w);
     if (fhat_in == fhat_out) return fail(c, LBM_ERR_ARG, "macrovars_drift_adj: the two adjoint arrays must be distinct");
-    const int nl = c->p.nl;
     if (!c->d_adj_terms)
         LBM_TRY(cuda_check(c, cudaMalloc(&c->d_adj_terms, (size_t)4 * c->rg.ncell() * sizeof(float)),
                            "cudaMalloc(macrovars adjoint terms)"));
     k_ref_macro_adj_terms<<<dim3((c->p.nx + 255) / 256, c->p.ny, c->p.nz), 256, 0, c->stream>>>(
-        c->d_adj_terms, rhohat, uhat, vhat, what, rho, u, v, w, c->rg);
-    const dim3 grd(c->p.ny + 2, c->p.nz + 2);
-    if (nl == 27) k_ref_macro_drift_adj<27><<<grd, 256, 0, c->stream>>>(fhat_in, fhat_out, c->d_adj_terms, c->rg);
-    else k_ref_macro_drift_adj<19><<<grd, 256, 0, c->stream>>>(fhat_in, fhat_out, c->d_adj_terms, c->rg);
-    k_ref_zero_interior<<<dim3(c->p.ny, c->p.nz), 256, 0, c->stream>>>(fhat_out, c->rg);
-    c->launches += 3;
-    LBM_LAUNCHED(c, "macrovars + drift adjoint");
-    return LBM_OK;
+        (float4*)c->d_adj_terms, rhohat, uhat, vhat, what, rho, u, v, w, c->rg);
+    c->launches++;
+    return c->p.nl == 27 ? drift_adj_launch<27, true>(c, fhat_in, fhat_out, (const float4*)c->d_adj_terms)
+                         : drift_adj_launch<19, true>(c, fhat_in, fhat_out, (const float4*)c->d_adj_terms);
 }
 
 int lbm_boundarycond_adj(lbm_ctx* c, float* f1hat, float* f2hat, float* uvelhat) {

@@ -237,13 +237,18 @@ struct DriftShape {
     int rs;        // row stride of the ring: room for a row, congruent to the global stride
 };
 template <int Q, typename R>
+int drift_row_stride(const RefGrid& g) {
+    using D = DriftTile<Q, R>;
+    return (D::WORDS + 1) * D::V + (int)(((long long)(g.nx + 2) * Q) % D::V);
+}
+// rows of g.nx cells, g.ny rows, g.nz planes of an array with one ghost cell at every end
+template <int Q, typename R>
 DriftShape drift_shape(const RefGrid& g, int slots) {
     using D = DriftTile<Q, R>;
     DriftShape d;
     const int nch = (g.nx + D::NI - 1) / D::NI;
     d.ni = (g.nx + nch - 1) / nch;
-    const int least = (D::WORDS + 1) * D::V;
-    d.rs = least + (int)(((long long)(g.nx + 2) * Q) % D::V);
+    d.rs = drift_row_stride<Q, R>(g);
     // segments of k: a block takes about ks + 4 plane times (two extra planes and the
     // first ones' latency); `slots` blocks run at a time
     const long long columns = (long long)nch * ((g.ny + D::TJ - 1) / D::TJ);
