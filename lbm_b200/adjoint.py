@@ -156,7 +156,9 @@ class FusedProbeProblem:
     steps, and for the first segment the imported state buffer (the input of
     step 0) with a snapshot after step 0.  Each segment is replayed from its
     snapshot, each step writing its state buffer into an array of its own
-    (``lbm_step_to``)."""
+    (``lbm_step_to``).  The last segment needs no replay: the forward's own steps
+    write their states into such arrays.  A step that a snapshot follows writes
+    its state straight into the snapshot."""
 
     def __init__(self, params: Params, probes, nsteps: int, blanking=None, checkpoint: int = 10):
         if params.storage != "f32":
@@ -173,10 +175,11 @@ class FusedProbeProblem:
         if blanking is not None:
             self.lbm.set_solids(blanking)
         self.ckpt = {}
+        self._last = None      # the states after the steps of the last segment, while they are kept
 
     def _import(self, f1, f2):
         L = self.lbm
-        R = [L.empty_s() for _ in range(4)]
+        R = [torch.empty(self.p.sshape, device="cuda") for _ in range(4)]   # macrovars writes every cell
         L.macrovars(*R, f1)
         L.state_import(f1, f2, *R)
         L.set_inflow(self.uvel)
@@ -185,17 +188,32 @@ class FusedProbeProblem:
         L = self.lbm
         self.uvel = uvel.contiguous()
         self.ckpt = {}
+        self._last = None
         self._import(f1, f2)
+        last = (self.nsteps - 1) // self.K * self.K      # first step of the last segment
+        states = []
         for n in range(self.nsteps):
-            if keep and n % self.K == 0 and n > 0:
-                self.ckpt[n] = L.snapshot()
+            snap = keep and (n + 1) % self.K == 0 and n + 1 < self.nsteps
+            into = None
             if keep and n == 0:
                 pre = L.state_scratch()
                 L.state_copy(pre)            # the imported f1: the input of step 0
-            L.step(1)
+            elif snap:
+                into = L.snapshot_scratch()
+            elif keep and n >= last:
+                into = L.state_scratch()
+            if into is None:
+                L.step(1)
+            else:
+                L.step_to(into)
             if keep and n == 0:
                 self.ckpt[0] = (pre, L.snapshot())   # and the state after step 0
-        R = [L.empty_s() for _ in range(4)]
+            if snap:
+                self.ckpt[n + 1] = L.snapshot(into)
+            if keep and n >= last:
+                states.append(self.ckpt[0][1] if n == 0 else into)
+        self._last = states if keep else None
+        R = [torch.empty(self.p.sshape, device="cuda") for _ in range(4)]    # get_macro writes every cell
         L.get_macro(*R)
         return torch.stack([R[q].reshape(-1)[self.pidx] for q in (1, 2, 3)], dim=1)
 
@@ -226,13 +244,23 @@ class FusedProbeProblem:
         rep.wait_stream(main)                # the forward's snapshots and the seed are written on main
         R.set_inflow(self.uvel)
         nsets = 2 if overlap else 1
-        sets = [[L.state_scratch() for _ in range(self.K)] for _ in range(nsets)]
+        sets = [None] * nsets                # arrays of a replayed segment, made when a replay first needs them
         released = [None] * nsets            # event: the adjoint is done with a set
 
         def replay(q):
             """The states of segment q: P[n - s] after step n, and the input of step s."""
             s, b = segs[q], q % nsets
             e = min(s + self.K, self.nsteps)
+            if q == 0 and self._last is not None:
+                return (self.ckpt[0][0] if s == 0 else self.ckpt[s]), self._last, None
+            if sets[b] is None:
+                # set 0 begins with the arrays the forward kept, whose segment is done by now
+                # (a second call then replays that one too)
+                sets[b] = []
+                if b == 0 and self._last is not None:
+                    sets[b] = [t for t in self._last if t is not self.ckpt[0][1]]
+                    self._last = None
+                sets[b] += [L.state_scratch() for _ in range(self.K - len(sets[b]))]
             P = list(sets[b][:e - s])
             with torch.cuda.stream(rep):
                 if released[b] is not None:
@@ -260,7 +288,8 @@ class FusedProbeProblem:
             b = q % nsets
             e = min(s + self.K, self.nsteps)
             first, P, ready = pending
-            main.wait_event(ready)
+            if ready is not None:
+                main.wait_event(ready)
             with torch.cuda.stream(main):
                 if e == self.nsteps:
                     L.state_adjoint_seed(A, P[e - s - 1], self.probes_dev, uhat_probes.float())
@@ -273,7 +302,7 @@ class FusedProbeProblem:
             released[b] = done
             if q + 1 < len(segs):
                 pending = replay(q + 1)
-        g = L.empty_f()
+        g = torch.empty(self.p.fshape, device="cuda")        # the export writes every cell
         L.state_adjoint_export(g, A)
         main.synchronize()
         del sets
@@ -281,6 +310,7 @@ class FusedProbeProblem:
 
     def close(self):
         self.ckpt = {}
+        self._last = None
         if getattr(self, "_rep", None) is not None:
             self._rep.close()
             self._rep = None

@@ -372,10 +372,15 @@ class Lbm:
         self._call("lbm_state_snapshot_bytes", ctypes.byref(n))
         return int(n.value)
 
+    def snapshot_scratch(self):
+        """An uninitialised array for :meth:`snapshot` (and for :meth:`step_to`, whose state
+        buffer is a snapshot's first part)."""
+        return torch.empty((self.snapshot_bytes() + 3) // 4, dtype=torch.float32, device="cuda")
+
     def snapshot(self, dst=None):
         """Device snapshot of the stepped state (allocated when ``dst`` is None)."""
         if dst is None:
-            dst = torch.empty((self.snapshot_bytes() + 3) // 4, dtype=torch.float32, device="cuda")
+            dst = self.snapshot_scratch()
         self._call("lbm_state_snapshot", _ptr(dst))
         return dst
 

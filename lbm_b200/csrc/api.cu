@@ -1410,7 +1410,8 @@ int lbm_state_snapshot(lbm_ctx* c, void* dst) {
     const SnapLayout L = snap_layout(c);
     char* d = static_cast<char*>(dst);
     const size_t nbuf = state_bytes_of(c);
-    LBM_TRY(cuda_check(c, cudaMemcpyAsync(d, c->buf[c->cur], nbuf, cudaMemcpyDeviceToDevice, c->stream), "snapshot"));
+    if (c->buf[c->cur] != dst)   // the last step may have written its state there (lbm_step_to)
+        LBM_TRY(cuda_check(c, cudaMemcpyAsync(d, c->buf[c->cur], nbuf, cudaMemcpyDeviceToDevice, c->stream), "snapshot"));
     pack_ghosts(c, d + L.buf, c->buf[1 - c->cur], false);
     if (c->fold) {
         const size_t nxg = (size_t)2 * c->p.nl * c->p.ny * c->p.nz * c->elem;
