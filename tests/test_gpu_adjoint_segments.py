@@ -1,0 +1,47 @@
+"""The fused gradient over every way its steps fall into segments: a single one, full and
+short last ones, one step each; with and without overlap, twice in a row, and from a
+forward run that kept another run's arrays before."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nsteps,K", [(1, 1), (2, 1), (5, 1), (3, 10), (4, 4), (8, 4), (9, 4), (11, 4), (13, 3)])
+def test_segments_give_the_percall_gradient(nsteps, K):
+    from lbm_b200 import Lbm, Params
+    from lbm_b200.adjoint import FusedProbeProblem, ProbeProblem, initial_state
+    p = Params(nx=20, ny=6, nz=8, nl=19, iturb_pos=2)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nsteps * 16 + K)
+    m = [torch.zeros(p.sshape, device="cuda") for _ in range(4)]
+    m[0][1:-1, 1:-1, 1:-1] = 1.0
+    for q in (1, 2, 3):
+        m[q][1:-1, 1:-1, 1:-1] = 0.03 * torch.randn((p.nz, p.ny, p.nx), device="cuda", generator=g)
+    uvel = torch.full((p.nz,), 0.05, device="cuda")
+    with Lbm(p) as L:
+        f1, f2 = initial_state(L, *m, uvel)
+        torch.cuda.synchronize()
+    f1 *= 1.0 + 5e-3 * torch.randn(f1.shape, device="cuda", generator=g)      # away from exact equilibrium
+    mask = torch.zeros(p.sshape, dtype=torch.int32, device="cuda")
+    mask[3:5, 3:5, 6:9] = 1
+    cells = np.array([[3, 2, 2], [15, 5, 7], [10, 3, 4], [20, 6, 8], [1, 1, 1]])
+    uhat = torch.randn((len(cells), 3), device="cuda", generator=g)
+    ref = ProbeProblem(p, cells, nsteps, blanking=mask, checkpoint=3)
+    ru = ref.forward(f1, f2, uvel)
+    rg, rv = ref.backward(uhat)
+    a = FusedProbeProblem(p, cells, nsteps, blanking=mask, checkpoint=K)
+    a.forward(f1 * 1.001, f2, uvel)              # another run's arrays are dropped
+    for _ in range(2):
+        u = a.forward(f1, f2, uvel)
+        assert float((u - ru).abs().max()) < 1e-6
+        for overlap in (True, True, False, False):
+            # the same sums in another order, some by atomics: within the two sweeps' distance (3e-5 of
+            # the largest entry, test_gpu_adjoint.py)
+            fg, fv = a.backward(uhat, overlap=overlap)
+            assert float((fg - rg).abs().max()) < 1e-4 * float(rg.abs().max())
+            assert float((fv - rv).abs().max()) < 1e-4 * float(rv.abs().max())
+    assert float((a.forward(f1, f2, uvel, keep=False) - ru).abs().max()) < 1e-6
+    a.close()
+    ref.close()
