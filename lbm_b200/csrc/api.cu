@@ -978,7 +978,8 @@ int lbm_create(lbm_ctx** out, const lbm_params* p) {
     const size_t g = (size_t)c->rg.ncell();
     chk(cudaMalloc(&c->d_macro, 4 * g * sizeof(float)), "cudaMalloc(macro)");
     chk(cudaMalloc(&c->d_uvel, (size_t)p->nz * sizeof(float)), "cudaMalloc(uvel)");
-    chk(cudaMalloc(&c->d_edge, (size_t)2 * p->nl * p->ny * p->nz * c->elem), "cudaMalloc(edge)");
+    const size_t edge_cell = (p->nl * c->elem + 15) / 16 * 16;   // EdgeCell
+    chk(cudaMalloc(&c->d_edge, (size_t)2 * p->ny * p->nz * edge_cell), "cudaMalloc(edge)");
     for (int b = 0; b < 2 && c->fold; ++b)
         chk(cudaMalloc(&c->d_xg[b], (size_t)2 * p->nl * p->ny * p->nz * c->elem), "cudaMalloc(x-ghost)");
     chk(cudaMalloc(&c->d_abl, (size_t)p->nz * sizeof(float)), "cudaMalloc(ablvisc)");

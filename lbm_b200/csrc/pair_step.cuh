@@ -410,15 +410,12 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
 template <int Q, typename S, bool ODD = false>
 __device__ __forceinline__ void pair_edge(const f2 (&fp)[Q], const StepArgs& a, int i, int j, int k) {
     if (i == 1 || (ODD ? i : i + 1) == a.g.nx) {
-        // the boundary kernel builds the inflow/outflow ghosts from these, read coalesced
-        const long long nyz = (long long)a.g.ny * a.g.nz;
+        // the boundary kernel builds the inflow/outflow ghosts from these
         const int side = (i == 1) ? 0 : 1, c = ODD ? 0 : side;
-        S* e = (S*)a.edge + (long long)side * Q * nyz + (long long)(k - 1) * a.g.ny + (j - 1);
+        float v[EdgeCell<Q, S>::N] = {};
 #pragma unroll
-        for (int l = 0; l < Q; ++l) {
-            if constexpr (sizeof(S) == 2) e[l * nyz] = __float2half_rn(comp(fp[l], c));   // already 2^8-scaled
-            else e[l * nyz] = comp(fp[l], c);
-        }
+        for (int l = 0; l < Q; ++l) v[l] = comp(fp[l], c);
+        edge_put<Q>(edge_at<Q, S>(a.edge, a.g, side, j, k), v);
     }
 }
 
@@ -465,11 +462,18 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
             *reinterpret_cast<__half2*>(reinterpret_cast<char*>(q) + a.soffb[l]) = h[l];
         }
         if (FOLD && (i == 1 || (!ODD && i + 1 == a.g.nx))) {
-            const long long nyz = (long long)a.g.ny * a.g.nz;
-            const int c = (i == 1) ? 0 : 1;
-            __half* e = (__half*)a.edge + (long long)c * Q * nyz + (long long)(k - 1) * a.g.ny + (j - 1);
+            constexpr int N = EdgeCell<Q, S>::N;
+            const unsigned half = (i == 1) ? 0x5410u : 0x7632u;   // the low or the high halves of two words
+            unsigned u[N / 2];
 #pragma unroll
-            for (int l = 0; l < Q; ++l) e[l * nyz] = c ? __high2half(h[l]) : __low2half(h[l]);
+            for (int l = 0; l < N / 2; ++l) {
+                const __half2 z = __float2half2_rn(0.0f);
+                const __half2 x = 2 * l < Q ? h[2 * l < Q ? 2 * l : 0] : z, y = 2 * l + 1 < Q ? h[2 * l + 1 < Q ? 2 * l + 1 : 0] : z;
+                u[l] = __byte_perm(*reinterpret_cast<const unsigned*>(&x), *reinterpret_cast<const unsigned*>(&y), half);
+            }
+            uint4* e = reinterpret_cast<uint4*>(edge_at<Q, S>(a.edge, a.g, i == 1 ? 0 : 1, j, k));
+#pragma unroll
+            for (int w = 0; w < EdgeCell<Q, S>::W; ++w) e[w] = make_uint4(u[4 * w], u[4 * w + 1], u[4 * w + 2], u[4 * w + 3]);
         }
     } else {
 #pragma unroll

@@ -74,7 +74,7 @@ struct alignas(16) StepArgs {
     const float* uvel;        // inflow profile uvel(nz)
     float rho0, cosd, sind;   // inflow constants (m_boundary_i_inflow_kernel.F90:35,71-73)
     int* d_it_rw;             // step counter, advanced by the boundary kernel
-    void* edge;               // post-collision populations at i=1 and i=nx: [side][l][k-1][j-1]
+    void* edge;               // post-collision populations at i=1 and i=nx: [side][k-1][j-1][EdgeCell::N]
     int peri;                 // periodic in i, j and k: the pair kernel writes the i ghosts
     int full_sector;          // x-ghost sectors hold nothing but the ghost and padding
     void* xg_dst;             // x-ghost columns of the buffer the step writes: [side][l][k-1][j-1]
@@ -151,6 +151,42 @@ struct PullLoop<Q, S, Q> {
 // a buffer's compact x-ghost array xg[side][l][k-1][j-1] (j, k interior).
 __device__ __forceinline__ long long xg_index(const SoaGrid& g, int Q, int side, int l, int j, int k) {
     return ((long long)(side * Q + l) * g.nz + (k - 1)) * g.ny + (j - 1);
+}
+
+// The edge array keeps a cell's Q values together, padded to whole 16-byte words: the
+// one thread of a row's end writes 5 to 7 of them (FP32), where a value each to
+// Q separate lines cost the warp Q stores and their addresses (step kernel, D3Q27
+// FP16 512x256x256 692 -> 681 us, FP32 128x64x64 27.7 -> 26.5; the boundary kernel
+// reads it 1 to 3 us slower).
+template <int Q, typename S>
+struct EdgeCell {
+    static constexpr int N = (Q * (int)sizeof(S) + 15) / 16 * 16 / (int)sizeof(S);
+    static constexpr int W = N * (int)sizeof(S) / 16;
+};
+// v: the cell's values as stored, padded with anything
+template <int Q>
+__device__ __forceinline__ void edge_put(float* e, const float (&v)[EdgeCell<Q, float>::N]) {
+#pragma unroll
+    for (int w = 0; w < EdgeCell<Q, float>::W; ++w)
+        reinterpret_cast<float4*>(e)[w] = make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
+}
+template <int Q>
+__device__ __forceinline__ void edge_put(__half* e, const float (&v)[EdgeCell<Q, __half>::N]) {
+    constexpr int N = EdgeCell<Q, __half>::N;
+    unsigned u[N / 2];
+#pragma unroll
+    for (int l = 0; l < N / 2; ++l) {
+        const __half2 h = __floats2half2_rn(v[2 * l], v[2 * l + 1]);
+        u[l] = *reinterpret_cast<const unsigned*>(&h);
+    }
+#pragma unroll
+    for (int w = 0; w < EdgeCell<Q, __half>::W; ++w)
+        reinterpret_cast<uint4*>(e)[w] = make_uint4(u[4 * w], u[4 * w + 1], u[4 * w + 2], u[4 * w + 3]);
+}
+// the values at edge cell (side, j, k)
+template <int Q, typename S>
+__device__ __forceinline__ S* edge_at(void* edge, const SoaGrid& g, int side, int j, int k) {
+    return (S*)edge + (((long long)side * g.nz + (k - 1)) * g.ny + (j - 1)) * EdgeCell<Q, S>::N;
 }
 
 // Store one 32-byte sector (two 16-byte vectors) holding v at element `slot`
@@ -235,12 +271,13 @@ template <int Q, typename S, int SIDE>
 __device__ __forceinline__ void bc_fold_xcol(S* f1, const StepArgs& a, int j, int k, long long cell) {
     const SoaGrid& g = a.g;
     const long long nyz = (long long)g.ny * g.nz;
-    const S* edge = (const S*)a.edge + (long long)SIDE * Q * nyz + cell;   // cell 1 (side 0) or nx (side 1)
+    constexpr int EN = EdgeCell<Q, S>::N;
+    const S* edge = (const S*)a.edge + ((long long)SIDE * nyz + cell) * EN;   // cell 1 (side 0) or nx (side 1)
     S* xg = (S*)a.xg_dst + (long long)SIDE * Q * nyz + cell;                 // xg_index(g, Q, SIDE, l, j, k)
     const int ig = SIDE ? g.nx + 1 : 0;   // the ghost column
-    S ev[Q];
+    __align__(16) S ev[EN];
 #pragma unroll
-    for (int l = 0; l < Q; ++l) ev[l] = edge[l * nyz];
+    for (int w = 0; w < EdgeCell<Q, S>::W; ++w) reinterpret_cast<uint4*>(ev)[w] = reinterpret_cast<const uint4*>(edge)[w];
     const float uu = SIDE ? 0.0f : a.uvel[k - 1];
     if (k == 1 || k == g.nz) {
         constexpr int NS = (Q == 27) ? 9 : 5;   // directions the pull reads at this ghost
@@ -317,10 +354,11 @@ __device__ __forceinline__ void bc_fold_xelem(S* f1, const StepArgs& a, long lon
     const long long cell = (long long)(k - 1) * g.ny + (j - 1);
     // inflow: directions with cx > 0 take the corrected value of their opposite
     const int ls = (cx > 0) ? c_opp[l] : l;
-    const float fin = Store<S>::to_f(edge[(long long)ls * nyz + cell]);
+    constexpr int EN = EdgeCell<Q, S>::N;
+    const float fin = Store<S>::to_f(edge[cell * EN + ls]);
     const S gin = Store<S>::from_f(inflow_value(fin, c_w[Q == 27 ? 1 : 0][ls], c_cx[ls], c_cy[ls], a.uvel[k - 1], a));
     // outflow: zero gradient
-    const S gout = edge[((long long)Q + l) * nyz + cell];
+    const S gout = edge[(nyz + cell) * EN + l];
     S* xg = (S*)a.xg_dst;
     xg[xg_index(g, Q, 0, l, j, k)] = gin;
     xg[xg_index(g, Q, 1, l, j, k)] = gout;
@@ -619,10 +657,10 @@ __global__ void __launch_bounds__(128, 8) k_step(const S* src, S* dst, StepArgs 
     for (int l = 0; l < Q; ++l) Store<S>::store(dst + (long long)l * g.dstride + o, fp[l]);
     if (WRAP && (i == 1 || i == g.nx)) {
         // the boundary kernel builds the inflow/outflow ghosts from these, read coalesced
-        const long long nyz = (long long)g.ny * g.nz;
-        S* e = (S*)a.edge + (i == 1 ? 0 : (long long)Q * nyz) + (long long)(k - 1) * g.ny + (j - 1);
+        float v[EdgeCell<Q, S>::N] = {};
 #pragma unroll
-        for (int l = 0; l < Q; ++l) e[l * nyz] = Store<S>::from_f(fp[l]);
+        for (int l = 0; l < Q; ++l) v[l] = fp[l] * store_scale<S>();
+        edge_put<Q>(edge_at<Q, S>(a.edge, g, i == 1 ? 0 : 1, j, k), v);
     }
 }
 
@@ -687,13 +725,10 @@ __device__ __forceinline__ void cell_update(float (&fp)[Q], S* __restrict__ dst,
     }
     if (WRAP && (i == 1 || i == a.g.nx)) {
         // the boundary kernel builds the inflow/outflow ghosts from these, read coalesced
-        const long long nyz = (long long)a.g.ny * a.g.nz;
-        S* e = (S*)a.edge + (i == 1 ? 0 : (long long)Q * nyz) + (long long)(k - 1) * a.g.ny + (j - 1);
+        float v[EdgeCell<Q, S>::N] = {};
 #pragma unroll
-        for (int l = 0; l < Q; ++l) {
-            if constexpr (sizeof(S) == 2) e[l * nyz] = __float2half_rn(fp[l]);
-            else e[l * nyz] = fp[l];
-        }
+        for (int l = 0; l < Q; ++l) v[l] = fp[l];
+        edge_put<Q>(edge_at<Q, S>(a.edge, a.g, i == 1 ? 0 : 1, j, k), v);
     }
 }
 
