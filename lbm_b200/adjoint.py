@@ -176,6 +176,7 @@ class FusedProbeProblem:
             self.lbm.set_solids(blanking)
         self.ckpt = {}
         self._last = None      # the states after the steps of the last segment, while they are kept
+        self._live = []        # the last two: the buffers that the context itself still holds
 
     def _import(self, f1, f2):
         L = self.lbm
@@ -213,6 +214,7 @@ class FusedProbeProblem:
             if keep and n >= last:
                 states.append(self.ckpt[0][1] if n == 0 else into)
         self._last = states if keep else None
+        self._live = states[-2:]
         R = [torch.empty(self.p.sshape, device="cuda") for _ in range(4)]    # get_macro writes every cell
         L.get_macro(*R)
         return torch.stack([R[q].reshape(-1)[self.pidx] for q in (1, 2, 3)], dim=1)
@@ -254,11 +256,12 @@ class FusedProbeProblem:
             if q == 0 and self._last is not None:
                 return (self.ckpt[0][0] if s == 0 else self.ckpt[s]), self._last, None
             if sets[b] is None:
-                # set 0 begins with the arrays the forward kept, whose segment is done by now
-                # (a second call then replays that one too)
+                # set 0 begins with the arrays the forward kept, whose segment is done by now (a
+                # second call then replays that one too), but for the context's own two
                 sets[b] = []
                 if b == 0 and self._last is not None:
-                    sets[b] = [t for t in self._last if t is not self.ckpt[0][1]]
+                    held = [self.ckpt[0][1]] + self._live
+                    sets[b] = [t for t in self._last if all(t is not h for h in held)]
                     self._last = None
                 sets[b] += [L.state_scratch() for _ in range(self.K - len(sets[b]))]
             P = list(sets[b][:e - s])
@@ -311,6 +314,7 @@ class FusedProbeProblem:
     def close(self):
         self.ckpt = {}
         self._last = None
+        self._live = []
         if getattr(self, "_rep", None) is not None:
             self._rep.close()
             self._rep = None

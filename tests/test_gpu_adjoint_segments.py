@@ -36,12 +36,18 @@ def test_segments_give_the_percall_gradient(nsteps, K):
     for _ in range(2):
         u = a.forward(f1, f2, uvel)
         assert float((u - ru).abs().max()) < 1e-6
+        end = [a.lbm.empty_s() for _ in range(4)]
+        a.lbm.get_macro(*end)
         for overlap in (True, True, False, False):
             # the same sums in another order, some by atomics: within the two sweeps' distance (3e-5 of
             # the largest entry, test_gpu_adjoint.py)
             fg, fv = a.backward(uhat, overlap=overlap)
             assert float((fg - rg).abs().max()) < 1e-4 * float(rg.abs().max())
             assert float((fv - rv).abs().max()) < 1e-4 * float(rv.abs().max())
+            if overlap:      # the forward's context still holds the state after the last step
+                now = [a.lbm.empty_s() for _ in range(4)]
+                a.lbm.get_macro(*now)
+                assert all(torch.equal(x, y) for x, y in zip(now, end))
     assert float((a.forward(f1, f2, uvel, keep=False) - ru).abs().max()) < 1e-6
     a.close()
     ref.close()
