@@ -232,39 +232,40 @@ __device__ __forceinline__ void collide_adj(const float (&fp)[Q], const float (&
 // stored in turn: 54 us for D3Q19 128x64x64, 2.5 TB/s).
 template <int Q>
 struct PostcollAdjTile {
+    static constexpr int T = 128;
     static constexpr int SC = 9;                                    // rho, u, v, w, tau and the four adjoints
-    static constexpr int STAGE = 2 * CellTile<Q, float>::BUF + SC * CELL_T;
+    static constexpr int STAGE = 2 * CellTile<Q, float, T>::BUF + SC * T;
     static constexpr size_t SMEM = 2 * STAGE * sizeof(float);
     static constexpr int BLOCKS = Q == 27 ? 3 : 4;
 };
 template <int Q>
-__global__ void __launch_bounds__(CELL_T, PostcollAdjTile<Q>::BLOCKS)
+__global__ void __launch_bounds__(PostcollAdjTile<Q>::T, PostcollAdjTile<Q>::BLOCKS)
     k_ref_postcoll_adj(float* fh, const float* f, const float* rho, const float* u, const float* v, const float* w,
                        const float* tau, const float* abl, float* rhoh, float* uh, float* vh, float* wh,
                        const int32_t* blank, RefGrid g, CollideParams cp, unsigned tp, unsigned ntiles) {
     using P = PostcollAdjTile<Q>;
-    constexpr int BUF = CellTile<Q, float>::BUF;
+    constexpr int T = P::T, BUF = CellTile<Q, float, T>::BUF;
     extern __shared__ __align__(16) unsigned char raw[];
-    __shared__ unsigned cells[CELL_T / 32];
+    __shared__ unsigned cells[T / 32];
     float* sm = reinterpret_cast<float*>(raw);
     const int tid = threadIdx.x;
     auto fetch = [&](unsigned t, int b) {
-        const TileAt a = tile_at<false>(g, t, tp);
+        const TileAt a = tile_at<false, T>(g, t, tp);
         float* s = sm + b * P::STAGE;
-        tile_fetch<Q>(s, f, a.c0, a.n);
-        tile_fetch<Q>(s + BUF, fh, a.c0, a.n);
+        tile_fetch<Q, T>(s, f, a.c0, a.n);
+        tile_fetch<Q, T>(s + BUF, fh, a.c0, a.n);
         if (tid < a.n) {
             s += 2 * BUF + tid;
             const long long c = a.c0 + tid;
             cp_async_elem(s, rho + c);
-            cp_async_elem(s + CELL_T, u + c);
-            cp_async_elem(s + 2 * CELL_T, v + c);
-            cp_async_elem(s + 3 * CELL_T, w + c);
-            cp_async_elem(s + 4 * CELL_T, tau + c);
-            cp_async_elem(s + 5 * CELL_T, rhoh + c);
-            cp_async_elem(s + 6 * CELL_T, uh + c);
-            cp_async_elem(s + 7 * CELL_T, vh + c);
-            cp_async_elem(s + 8 * CELL_T, wh + c);
+            cp_async_elem(s + T, u + c);
+            cp_async_elem(s + 2 * T, v + c);
+            cp_async_elem(s + 3 * T, w + c);
+            cp_async_elem(s + 4 * T, tau + c);
+            cp_async_elem(s + 5 * T, rhoh + c);
+            cp_async_elem(s + 6 * T, uh + c);
+            cp_async_elem(s + 7 * T, vh + c);
+            cp_async_elem(s + 8 * T, wh + c);
         }
     };
     fetch(blockIdx.x, 0);
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(CELL_T, PostcollAdjTile<Q>::BLOCKS)
     for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
         if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
         cp_async_commit();
-        const TileAt a = tile_at<false>(g, t, tp);
+        const TileAt a = tile_at<false, T>(g, t, tp);
         const unsigned i = (a.q0 + tid) % (unsigned)(g.nx + 2);
         const bool inner = tid < a.n && i >= 1 && i <= (unsigned)g.nx;
         const unsigned mask = __ballot_sync(0xffffffffu, inner);
@@ -302,17 +303,17 @@ __global__ void __launch_bounds__(CELL_T, PostcollAdjTile<Q>::BLOCKS)
                 }
             }
             float rr = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-            collide_adj<Q>(fp, gh, sc[0], sc[CELL_T], sc[2 * CELL_T], sc[3 * CELL_T], cp, abl ? abl[a.k - 1] : 0.0f,
-                           sc[4 * CELL_T], out, rr, ux, uy, uz);
-            rhoh[c] = sc[5 * CELL_T] + rr;
-            uh[c] = sc[6 * CELL_T] + ux;
-            vh[c] = sc[7 * CELL_T] + uy;
-            wh[c] = sc[8 * CELL_T] + uz;
+            collide_adj<Q>(fp, gh, sc[0], sc[T], sc[2 * T], sc[3 * T], cp, abl ? abl[a.k - 1] : 0.0f,
+                           sc[4 * T], out, rr, ux, uy, uz);
+            rhoh[c] = sc[5 * T] + rr;
+            uh[c] = sc[6 * T] + ux;
+            vh[c] = sc[7 * T] + uy;
+            wh[c] = sc[8 * T] + uz;
 #pragma unroll
             for (int l = 0; l < Q; ++l) sg[l] = out[l];
         }
         const bool whole = __syncthreads_and(inner);
-        tile_put<Q>(tile + BUF, fh, a.c0, a.n, cells, whole);
+        tile_put<Q, T>(tile + BUF, fh, a.c0, a.n, cells, whole);
         __syncthreads();
     }
 }

@@ -98,12 +98,12 @@ int lbm_postcoll_adj(lbm_ctx* c, float* fhat, const float* f, const float* tau, 
         return fail(c, LBM_ERR_UNSUPPORTED, "postcoll_adj: the adjoint covers the regularized collision (ihrr = 1)");
     // with Vreman the forward computes tau itself; any array stands in for the unused input
     const float* t = tau ? tau : rho;
-    const unsigned tp = plane_tiles(c->rg), nt = tp * (unsigned)c->p.nz;
+    const unsigned tp = plane_tiles(c->rg, PostcollAdjTile<27>::T), nt = tp * (unsigned)c->p.nz;   // the same T for both
     if (c->p.nl == 27)
-        return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<27>, PostcollAdjTile<27>::SMEM,
+        return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<27>, PostcollAdjTile<27>::T, PostcollAdjTile<27>::SMEM,
                             PostcollAdjTile<27>::BLOCKS, nt, fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
                             blanking, c->rg, c->cp, tp);
-    return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<19>, PostcollAdjTile<19>::SMEM,
+    return tiled_launch(c, "postcoll adjoint", k_ref_postcoll_adj<19>, PostcollAdjTile<19>::T, PostcollAdjTile<19>::SMEM,
                         PostcollAdjTile<19>::BLOCKS, nt, fhat, f, rho, u, v, w, t, ablvisc, rhohat, uhat, vhat, what,
                         blanking, c->rg, c->cp, tp);
 }

@@ -779,11 +779,11 @@ int fequil3_run(lbm_ctx* c, R* feq, const R* rho, const R* u, const R* v, const 
 
 // a tiled kernel: `blocks` resident per SM walk the tiles
 template <typename... KArgs, typename... Args>
-int tiled_launch(lbm_ctx* c, const char* what, void (*kern)(KArgs...), size_t smem, int blocks, unsigned ntiles,
-                 Args... args) {
+int tiled_launch(lbm_ctx* c, const char* what, void (*kern)(KArgs...), int threads, size_t smem, int blocks,
+                 unsigned ntiles, Args... args) {
     LBM_TRY(cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), what));
     const unsigned grid = std::min(ntiles, (unsigned)(c->nsm * blocks));
-    kern<<<grid, CELL_T, smem, c->stream>>>(args..., ntiles);
+    kern<<<grid, threads, smem, c->stream>>>(args..., ntiles);
     c->launches++;
     LBM_LAUNCHED(c, what);
     return LBM_OK;
@@ -792,8 +792,8 @@ int tiled_launch(lbm_ctx* c, const char* what, void (*kern)(KArgs...), size_t sm
 template <int Q, typename R>
 int postcoll_launch(lbm_ctx* c, R* f, R* tau, const R* rho, const R* u, const R* v, const R* w, const R* abl) {
     using P = PostcollTile<Q, R>;
-    const unsigned tp = plane_tiles(c->rg);
-    return tiled_launch(c, "postcoll", k_ref_postcoll<Q, R>, P::SMEM, P::BLOCKS, tp * (unsigned)c->p.nz, f, tau, rho, u, v,
+    const unsigned tp = plane_tiles(c->rg, P::T);
+    return tiled_launch(c, "postcoll", k_ref_postcoll<Q, R>, P::T, P::SMEM, P::BLOCKS, tp * (unsigned)c->p.nz, f, tau, rho, u, v,
                         w, abl, c->rg, cp_of<R>(c), tp);
 }
 template <typename R>
@@ -824,7 +824,7 @@ int drift_run(lbm_ctx* c, R* f, const R* feq) {
 template <int Q, typename R>
 int macrovars_launch(lbm_ctx* c, R* rho, R* u, R* v, R* w, const R* f) {
     using P = MacroTile<Q, R>;
-    return tiled_launch(c, "macrovars", k_ref_macrovars<Q, R>, P::SMEM, P::BLOCKS, all_tiles(c->rg), rho, u, v, w, f,
+    return tiled_launch(c, "macrovars", k_ref_macrovars<Q, R>, P::T, P::SMEM, P::BLOCKS, all_tiles(c->rg, P::T), rho, u, v, w, f,
                         c->rg);
 }
 template <typename R>

@@ -122,41 +122,48 @@ __global__ void __launch_bounds__(128) k_ref_fequil3(R* feq, const R* rho, const
 // Shared memory and resident blocks of the tiled kernels: two tile buffers with
 // `scalars` values per cell each; as many blocks as fit an SM, up to a cap on
 // their registers.
+// T: postcoll reads, computes and writes between three barriers, so more, smaller blocks
+// serve it where a block of 128 fills much of an SM: D3Q27 FP32 256x128x128 195 us in
+// tiles of 64 cells and 207 in tiles of 128, D3Q19 FP64 192x96x96 106 and 117; the
+// smaller D3Q19 FP32 tiles lose, 27.4 and 25.7 for 128x64x64.
 template <int Q, typename R>
 struct PostcollTile {
+    static constexpr int T = (sizeof(R) == 4 && Q == 19) ? 128 : 64;
     static constexpr int SC = 5;                                   // rho, u, v, w, tau
-    static constexpr int STAGE = CellTile<Q, R>::BUF + SC * CELL_T;    // elements of one of the two stages
+    static constexpr int STAGE = CellTile<Q, R, T>::BUF + SC * T;   // elements of one of the two stages
     static constexpr size_t SMEM = 2 * STAGE * sizeof(R);
-    static constexpr int BLOCKS = sizeof(R) == 4 ? (Q == 27 ? 6 : 7) : (Q == 27 ? 3 : 4);
+    static constexpr int BLOCKS = sizeof(R) == 4 ? (Q == 27 ? 12 : 7) : (Q == 27 ? 6 : 8);
 };
 template <int Q, typename R>
 struct MacroTile {
-    static constexpr int STAGE = CellTile<Q, R>::BUF;
+    static constexpr int T = 128;
+    static constexpr int STAGE = CellTile<Q, R, T>::BUF;
     static constexpr size_t SMEM = 2 * STAGE * sizeof(R);
     static constexpr int BLOCKS = sizeof(R) == 4 ? (Q == 27 ? 7 : 10) : (Q == 27 ? 4 : 5);
 };
 
 // postcoll: collide interior cells in place with the given moments (m_postcoll_kernel.F90:7-255)
 template <int Q, typename R = float>
-__global__ void __launch_bounds__(CELL_T, PostcollTile<Q, R>::BLOCKS)
+__global__ void __launch_bounds__(PostcollTile<Q, R>::T, PostcollTile<Q, R>::BLOCKS)
     k_ref_postcoll(R* f, R* tau, const R* rho, const R* u, const R* v, const R* w, const R* abl, RefGrid g,
                    CollideParamsT<R> cp, unsigned tp, unsigned ntiles) {
     using P = PostcollTile<Q, R>;
+    constexpr int T = P::T;
     extern __shared__ __align__(16) unsigned char raw[];
-    __shared__ unsigned cells[CELL_T / 32];
+    __shared__ unsigned cells[T / 32];
     R* sm = reinterpret_cast<R*>(raw);
     const int tid = threadIdx.x;
     auto fetch = [&](unsigned t, int b) {
-        const TileAt a = tile_at<false>(g, t, tp);
-        tile_fetch<Q>(sm + b * P::STAGE, f, a.c0, a.n);
+        const TileAt a = tile_at<false, T>(g, t, tp);
+        tile_fetch<Q, T>(sm + b * P::STAGE, f, a.c0, a.n);
         if (tid < a.n) {
-            R* s = sm + b * P::STAGE + CellTile<Q, R>::BUF + tid;
+            R* s = sm + b * P::STAGE + CellTile<Q, R, T>::BUF + tid;
             const long long c = a.c0 + tid;
             cp_async_elem(s, rho + c);
-            cp_async_elem(s + CELL_T, u + c);
-            cp_async_elem(s + 2 * CELL_T, v + c);
-            cp_async_elem(s + 3 * CELL_T, w + c);
-            cp_async_elem(s + 4 * CELL_T, tau + c);
+            cp_async_elem(s + T, u + c);
+            cp_async_elem(s + 2 * T, v + c);
+            cp_async_elem(s + 3 * T, w + c);
+            cp_async_elem(s + 4 * T, tau + c);
         }
     };
     fetch(blockIdx.x, 0);
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(CELL_T, PostcollTile<Q, R>::BLOCKS)
     for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
         if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
         cp_async_commit();
-        const TileAt a = tile_at<false>(g, t, tp);
+        const TileAt a = tile_at<false, T>(g, t, tp);
         const unsigned i = (a.q0 + tid) % (unsigned)(g.nx + 2);
         const bool inner = tid < a.n && i >= 1 && i <= (unsigned)g.nx;
         const unsigned mask = __ballot_sync(0xffffffffu, inner);
@@ -175,7 +182,7 @@ __global__ void __launch_bounds__(CELL_T, PostcollTile<Q, R>::BLOCKS)
         R* tile = sm + b * P::STAGE;
         if (inner) {
             R* s = tile + phase_of(f + a.c0 * Q) + tid * Q;
-            const R* sc = tile + CellTile<Q, R>::BUF + tid;
+            const R* sc = tile + CellTile<Q, R, T>::BUF + tid;
             R fp[Q];
 #pragma unroll
             for (int l = 0; l < Q; ++l) fp[l] = s[l] - lat_w<Q, R>(l);
@@ -184,14 +191,14 @@ __global__ void __launch_bounds__(CELL_T, PostcollTile<Q, R>::BLOCKS)
             TurbInT<R> tb;
             tb.on = false;
             tb.dux = tb.duy = tb.duz = R(0);
-            const R tnew = collide<Q>(fp, m, r - R(1.0), r, sc[CELL_T], sc[2 * CELL_T], sc[3 * CELL_T], cp,
-                                      abl ? abl[a.k - 1] : R(0.0), sc[4 * CELL_T], false, tb);
+            const R tnew = collide<Q>(fp, m, r - R(1.0), r, sc[T], sc[2 * T], sc[3 * T], cp,
+                                      abl ? abl[a.k - 1] : R(0.0), sc[4 * T], false, tb);
             if (cp.ivreman) tau[a.c0 + tid] = tnew;
 #pragma unroll
             for (int l = 0; l < Q; ++l) s[l] = fp[l] + lat_w<Q, R>(l);
         }
         const bool whole = __syncthreads_and(inner);
-        tile_put<Q>(tile, f, a.c0, a.n, cells, whole);
+        tile_put<Q, T>(tile, f, a.c0, a.n, cells, whole);
         __syncthreads();
     }
 }
@@ -340,15 +347,16 @@ __global__ void __launch_bounds__(DriftTile<Q, R>::T, DriftTile<Q, R>::BLOCKS)
 
 // macrovars over the ghost-inclusive grid, summation order of m_macrovars_kernel.F90:35-49
 template <int Q, typename R = float>
-__global__ void __launch_bounds__(CELL_T, MacroTile<Q, R>::BLOCKS)
+__global__ void __launch_bounds__(MacroTile<Q, R>::T, MacroTile<Q, R>::BLOCKS)
     k_ref_macrovars(R* rho, R* u, R* v, R* w, const R* f, RefGrid g, unsigned ntiles) {
     using P = MacroTile<Q, R>;
+    constexpr int T = P::T;
     extern __shared__ __align__(16) unsigned char raw[];
     R* sm = reinterpret_cast<R*>(raw);
     const int tid = threadIdx.x;
     auto fetch = [&](unsigned t, int b) {
-        const TileAt a = tile_at<true>(g, t, 0);
-        tile_fetch<Q>(sm + b * P::STAGE, f, a.c0, a.n);
+        const TileAt a = tile_at<true, T>(g, t, 0);
+        tile_fetch<Q, T>(sm + b * P::STAGE, f, a.c0, a.n);
     };
     fetch(blockIdx.x, 0);
     cp_async_commit();
@@ -356,7 +364,7 @@ __global__ void __launch_bounds__(CELL_T, MacroTile<Q, R>::BLOCKS)
     for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x, b ^= 1) {
         if (t + gridDim.x < ntiles) fetch(t + gridDim.x, b ^ 1);
         cp_async_commit();
-        const TileAt a = tile_at<true>(g, t, 0);
+        const TileAt a = tile_at<true, T>(g, t, 0);
         cp_async_wait<1>();
         __syncthreads();
         if (tid < a.n) {

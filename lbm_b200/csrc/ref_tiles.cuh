@@ -51,19 +51,18 @@ __device__ __forceinline__ void run_load_word(R* sm, const R* g, int ph, int n, 
     }
 }
 
-// ---- tiles of CELL_T consecutive cells --------------------------------------------
+// ---- tiles of T consecutive cells -------------------------------------------------
 //
-// The cell-wise kernels walk an array in tiles of CELL_T consecutive cells, a
+// The cell-wise kernels walk an array in tiles of T consecutive cells, a
 // thread per cell, in blocks that stay on their SM and fetch the next tile (and
 // its scalars) while they work on the current one.  Tiles run through the rows
 // j = 1..ny of a plane without regard to row ends (ALL: through the whole
 // array), so short rows leave no thread idle; the i ghosts they pass over are
 // read and never written.
-#define CELL_T 128
-template <int Q, typename R>
+template <int Q, typename R, int T>
 struct CellTile {
     static constexpr int V = word_elems<R>();
-    static constexpr int WORDS = (CELL_T * Q + 2 * (V - 1)) / V;   // words a tile may touch
+    static constexpr int WORDS = (T * Q + 2 * (V - 1)) / V;   // words a tile may touch
     static constexpr int BUF = (WORDS + 1) * V;                    // elements of a tile buffer
 };
 
@@ -74,44 +73,44 @@ struct TileAt {
     int k;             // plane (interior tiles)
     unsigned q0;       // first cell's index in the plane's rows j = 1..ny (interior tiles)
 };
-template <bool ALL>
+template <bool ALL, int T>
 __device__ __forceinline__ TileAt tile_at(const RefGrid& g, unsigned t, unsigned tp) {
     TileAt a;
     if (ALL) {
-        a.c0 = (long long)t * CELL_T;
-        a.n = (int)min((long long)CELL_T, g.ncell() - a.c0);
+        a.c0 = (long long)t * T;
+        a.n = (int)min((long long)T, g.ncell() - a.c0);
         a.k = 0;
         a.q0 = 0;
     } else {
         const unsigned per_plane = (unsigned)(g.nx + 2) * (unsigned)g.ny, k = t / tp;
-        a.q0 = (t - k * tp) * CELL_T;
+        a.q0 = (t - k * tp) * T;
         a.k = (int)k + 1;
-        a.n = (int)min((unsigned)CELL_T, per_plane - a.q0);
+        a.n = (int)min((unsigned)T, per_plane - a.q0);
         a.c0 = g.cell(0, 1, a.k) + a.q0;
     }
     return a;
 }
 // tiles of a plane's interior rows, and of the whole array
-inline unsigned plane_tiles(const RefGrid& g) { return ((unsigned)(g.nx + 2) * (unsigned)g.ny + CELL_T - 1) / CELL_T; }
-inline unsigned all_tiles(const RefGrid& g) { return (unsigned)((g.ncell() + CELL_T - 1) / CELL_T); }
+inline unsigned plane_tiles(const RefGrid& g, int T) { return ((unsigned)(g.nx + 2) * (unsigned)g.ny + T - 1) / T; }
+inline unsigned all_tiles(const RefGrid& g, int T) { return (unsigned)((g.ncell() + T - 1) / T); }
 
 // the n cells from c0 on to a tile buffer; their first element lands at phase_of(f + c0 Q)
-template <int Q, typename R>
+template <int Q, int T, typename R>
 __device__ __forceinline__ void tile_fetch(R* sm, const R* f, long long c0, int n) {
     const R* g = f + c0 * Q;
     const int ph = phase_of(g);
-    for (int w = threadIdx.x; w < CellTile<Q, R>::WORDS; w += CELL_T) run_load_word(sm, g, ph, n * Q, w);
+    for (int w = threadIdx.x; w < CellTile<Q, R, T>::WORDS; w += T) run_load_word(sm, g, ph, n * Q, w);
 }
 
-// a tile buffer back to the cells whose bit in `cells` (CELL_T / 32 words of shared
+// a tile buffer back to the cells whose bit in `cells` (T / 32 words of shared
 // memory) is set; whole: all of them are
-template <int Q, typename R>
+template <int Q, int T, typename R>
 __device__ __forceinline__ void tile_put(const R* sm, R* f, long long c0, int n, const unsigned* cells, bool whole) {
     constexpr int V = word_elems<R>();
     R* g = f + c0 * Q;
     const int ph = phase_of(g), m = n * Q;
     auto on = [&](int e) { const int c = e / Q; return (cells[c >> 5] >> (c & 31)) & 1u; };
-    for (int w = threadIdx.x; w < CellTile<Q, R>::WORDS; w += CELL_T) {
+    for (int w = threadIdx.x; w < CellTile<Q, R, T>::WORDS; w += T) {
         const int e = w * V - ph;
         if (e >= 0 && e + V <= m && (whole || (on(e) && on(e + V - 1)))) {
             *reinterpret_cast<uint4*>(g + e) = *reinterpret_cast<const uint4*>(sm + ph + e);
