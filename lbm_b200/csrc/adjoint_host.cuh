@@ -232,13 +232,21 @@ int lbm_state_adjoint_step(lbm_ctx* c, float* W, float* A, const void* P, int32_
     const float* Pf = static_cast<const float*>(P);
     const uint8_t* sol = c->d_solid;
     const float* abl = c->d_abl;
+    AdjOffsets off;
+    const long long plane = (long long)g.pitch * (g.ny + 2);
+    for (int l = 0; l < 27; ++l) {
+        const long long d = lat_cx(l) + (long long)lat_cy(l) * g.pitch + (long long)lat_cz(l) * plane;
+        off.own[l] = 4 * (l * g.dstride);
+        off.pull[l] = 4 * (l * g.dstride - d);
+        off.push[l] = 4 * (l * g.dstride + d);
+    }
     cudaError_t r;
     if (Q == 27)
-        r = pull ? launch_pdl(k_sadj_cell<27, true>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl)
-                 : launch_pdl(k_sadj_cell<27, false>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl);
+        r = pull ? launch_pdl(k_sadj_cell<27, true>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl, off)
+                 : launch_pdl(k_sadj_cell<27, false>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl, off);
     else
-        r = pull ? launch_pdl(k_sadj_cell<19, true>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl)
-                 : launch_pdl(k_sadj_cell<19, false>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl);
+        r = pull ? launch_pdl(k_sadj_cell<19, true>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl, off)
+                 : launch_pdl(k_sadj_cell<19, false>, inner, dim3(128), c->stream, W, A, Pf, g, wrap, awrap, sol, c->cp, abl, off);
     LBM_TRY(cuda_check(c, r, "state adjoint: collision"));
     c->launches++;
     LBM_LAUNCHED(c, "state adjoint: collision");

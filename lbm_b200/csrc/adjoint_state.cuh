@@ -246,28 +246,44 @@ __global__ void __launch_bounds__(32) k_sadj_xface(float* __restrict__ W, const 
 // awrap: the adjoint arrays read their j ghost rows as rows ny and 1 (SoaAdjAcc).
 // ROWS: the row is j = 1 or ny, where periodic j wraps (otherwise the wrap
 // adjustments of every address are compiled out).
+// off: byte offsets of direction l from a cell, constant operands of the loads and
+// stores (computing each 64-bit offset took a quarter of the kernel's 1,178
+// instructions a cell, which bind it: D3Q19 256x128x128 197 -> 177 us alone).
+struct AdjOffsets {
+    long long own[27], pull[27], push[27];   // its entry, its pull source, its push target
+};
+__device__ __forceinline__ const float* at_bytes(const float* p, long long off) {
+    return reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + off);
+}
 template <int Q, bool PULL, bool ROWS>
 __device__ __forceinline__ void sadj_cell(float* __restrict__ W, const float* __restrict__ A,
                                           const float* __restrict__ P, const SoaGrid& g, int wrap_, int awrap_,
                                           const uint8_t* __restrict__ solid, const CollideParams& cp,
-                                          const float* __restrict__ abl, int i, int j, int k) {
+                                          const float* __restrict__ abl, int i, int j, int k, const AdjOffsets& off) {
     const int wrap = ROWS ? wrap_ : 0, awrap = ROWS ? awrap_ : 0;
-    const long long o = g.off(i, j, k);
+    const long long o = g.off(i, j, k), wrapd = (long long)g.ny * g.pitch;
     float fp[Q], gh[Q];
-    if (PULL) {
-        PullMacro<Q, float, 0>::run(fp, P, g, o, j, wrap != 0);
-    } else {
+    float* w0 = W + o;
+    {
+        // pull sources lie in row j - 1 (cy > 0) and j + 1 (cy < 0), push targets the other way
+        const float* p0 = P + o;
+        const float* pp = (wrap && j == 1) ? p0 + wrapd : p0;
+        const float* pm = (wrap && j == g.ny) ? p0 - wrapd : p0;
+        const float* a0 = A + o;
+        const float* ap = (awrap && j == g.ny) ? a0 - wrapd : a0;
+        const float* am = (awrap && j == 1) ? a0 + wrapd : a0;
 #pragma unroll
-        for (int l = 0; l < Q; ++l) fp[l] = P[(long long)l * g.dstride + o];
+        for (int l = 0; l < Q; ++l)
+            fp[l] = PULL ? *at_bytes(lat_cy(l) > 0 ? pp : (lat_cy(l) < 0 ? pm : p0), off.pull[l]) : *at_bytes(p0, off.own[l]);
+#pragma unroll
+        for (int l = 0; l < Q; ++l) gh[l] = *at_bytes(lat_cy(l) > 0 ? ap : (lat_cy(l) < 0 ? am : a0), off.push[l]);
     }
     const bool wr = awrap != 0;
-#pragma unroll
-    for (int l = 0; l < Q; ++l) gh[l] = A[(long long)l * g.dstride + o + push_delta(g, l, j, wr)];
     if (near_shell(g, i, j, k, wr)) {
 #pragma unroll
         for (int l = 0; l < Q; ++l) {
             const int jt = wr ? wrapj(j + lat_cy(l), g.ny) : j + lat_cy(l);
-            gh[l] = (interior(g, i + lat_cx(l), jt, k + lat_cz(l)) ? gh[l] : 0.0f) + W[(long long)l * g.dstride + o];
+            gh[l] = (interior(g, i + lat_cx(l), jt, k + lat_cz(l)) ? gh[l] : 0.0f) + *at_bytes(w0, off.own[l]);
         }
     }
     if (solid && solid[((long long)(k - 1) * g.ny + (j - 1)) * g.nx + (i - 1)]) {
@@ -289,7 +305,8 @@ __device__ __forceinline__ void sadj_cell(float* __restrict__ W, const float* __
     // opposite pair (l, l+1): E = s0h + rh - a.u + c c : a_h, O = c . a
     const float ax = uxh * irho, ay = uyh * irho, az = uzh * irho;
     const float E0 = c.s0h + rh - (ax * ux + ay * uy + az * uz);
-    W[o] = E0;
+    auto put = [&](int l, float v) { *const_cast<float*>(at_bytes(w0, off.own[l])) = v; };
+    put(0, E0);
 #pragma unroll
     for (int l = 1; l < Q; l += 2) {
         const int cx = lat_cx(l), cy = lat_cy(l), cz = lat_cz(l);
@@ -303,8 +320,8 @@ __device__ __forceinline__ void sadj_cell(float* __restrict__ W, const float* __
         macc(O, cx, ax);
         macc(O, cy, ay);
         macc(O, cz, az);
-        W[(long long)l * g.dstride + o] = E + O;
-        W[(long long)(l + 1) * g.dstride + o] = E - O;
+        put(l, E + O);
+        put(l + 1, E - O);
     }
 }
 
@@ -312,13 +329,13 @@ template <int Q, bool PULL>
 __global__ void __launch_bounds__(128) k_sadj_cell(float* __restrict__ W, const float* __restrict__ A,
                                                    const float* __restrict__ P, SoaGrid g, int wrap, int awrap,
                                                    const uint8_t* __restrict__ solid, CollideParams cp,
-                                                   const float* __restrict__ abl) {
+                                                   const float* __restrict__ abl, const AdjOffsets off) {
     pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y + 1, k = blockIdx.z + 1;
     if (i > g.nx) return;
-    if (j == 1 || j == g.ny) sadj_cell<Q, PULL, true>(W, A, P, g, wrap, awrap, solid, cp, abl, i, j, k);
-    else sadj_cell<Q, PULL, false>(W, A, P, g, wrap, awrap, solid, cp, abl, i, j, k);
+    if (j == 1 || j == g.ny) sadj_cell<Q, PULL, true>(W, A, P, g, wrap, awrap, solid, cp, abl, i, j, k, off);
+    else sadj_cell<Q, PULL, false>(W, A, P, g, wrap, awrap, solid, cp, abl, i, j, k, off);
 }
 
 // loss seed: A(l, x_p) += d(u, v, w)(x_p)/df_l^T uhat_p at the probe cells, where
