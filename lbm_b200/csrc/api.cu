@@ -697,7 +697,8 @@ int step_dispatch(lbm_ctx* c) {
 template <int Q, typename S>
 void launch_import(lbm_ctx* c, const float* ref, int b) {
     const SoaGrid& g = c->sg;
-    k_import<Q, S><<<dim3((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2), 128, 0, c->stream>>>(ref, (S*)c->buf[b], g);
+    k_import<Q, S><<<dim3((g.nx + 2 + 127) / 128, g.ny + 2, g.nz + 2), 128, 0, c->stream>>>(ref, (S*)c->buf[b], g,
+                                                                                             pull_offsets(c));
     c->launches++;
     if (c->fold) launch_gather_xg<Q, S>(c, b);
 }

@@ -795,41 +795,6 @@ __global__ void k_bump_step(int* d_it) {
     if (threadIdx.x == 0 && blockIdx.x == 0) *d_it += 1;
 }
 
-// Reference layout (absolute FP32) -> state (offsets in S).  One block per
-// (row, chunk of 128 cells); the row is staged through shared memory so both
-// the strided reference reads and the per-direction writes are coalesced.
-template <int Q, typename S>
-__global__ void __launch_bounds__(128) k_import(const float* __restrict__ ref, S* __restrict__ dst, SoaGrid g) {
-    __shared__ float sm[128 * Q];
-    const int i0 = blockIdx.x * 128;
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int n = min(128, g.nx + 2 - i0);
-    if (n <= 0) return;
-    const long long base = ((long long)i0 + (long long)(g.nx + 2) * ((long long)j + (long long)(g.ny + 2) * k)) * Q;
-    // eight independent loads in flight per thread before their shared-memory stores
-    const int m = n * Q;
-    for (int e0 = threadIdx.x; e0 < m; e0 += blockDim.x * 8) {
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int e = e0 + u * blockDim.x;
-            if (e < m) v[u] = ref[base + e];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int e = e0 + u * blockDim.x;
-            if (e < m) sm[e] = v[u];
-        }
-    }
-    __syncthreads();
-    const int t = threadIdx.x;
-    if (t < n) {
-        const long long o = g.off(i0 + t, j, k);
-#pragma unroll
-        for (int l = 0; l < Q; ++l) dst[(long long)l * g.dstride + o] = Store<S>::from_f(sm[t * Q + l] - lat_w<Q>(l));
-    }
-}
-
 template <int Q, typename S, int L>
 struct PullMacro {
     static __device__ __forceinline__ void run(float (&fp)[Q], const S* src, const SoaGrid& g, long long o, int j,
@@ -849,6 +814,32 @@ struct PullMacro<Q, S, Q> {
 struct PullOffsets {
     long long poffb[27], soffb[27];
 };
+
+// Reference layout (absolute FP32) -> state (offsets in S).  One block per
+// (row, chunk of 128 cells); the row is staged through shared memory, in whole
+// 16-byte words that are all in flight at once, so both the strided reference
+// reads and the per-direction writes are coalesced.
+template <int Q, typename S>
+__global__ void __launch_bounds__(128) k_import(const float* __restrict__ ref, S* __restrict__ dst, SoaGrid g,
+                                                const PullOffsets off) {
+    __shared__ __align__(16) float sm[128 * Q + 4];
+    const int i0 = blockIdx.x * 128;
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int n = min(128, g.nx + 2 - i0);
+    if (n <= 0) return;
+    const float* src = ref + ((long long)i0 + (long long)(g.nx + 2) * ((long long)j + (long long)(g.ny + 2) * k)) * Q;
+    const int ph = phase_of(src), m = n * Q, t = threadIdx.x;
+    for (int w = t; w * 4 < ph + m; w += 128) run_load_word(sm, src, ph, m, w);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (t < n) {
+        char* p = reinterpret_cast<char*>(dst + g.off(i0 + t, j, k));
+        const float* v = sm + ph + t * Q;
+#pragma unroll
+        for (int l = 0; l < Q; ++l) *reinterpret_cast<S*>(p + off.soffb[l]) = Store<S>::from_f(v[l] - lat_w<Q>(l));
+    }
+}
 
 // A chunk of n cells (one thread each, row (j,k), first cell i0) of the
 // reference layout from a tile staged at sm[t Q + l + phase]: whole 16-byte

@@ -47,3 +47,31 @@ def test_export_matches_percall(nx, ny, nz, codes, nl, storage):
     e1, e2 = a.state()
     a.lbm.state_export(f1, f1)
     assert torch.equal(f1, e2)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("nl", [19, 27])
+@pytest.mark.parametrize("nx", [5, 126, 127, 200])
+def test_import_from_any_alignment(nx, nl, storage):
+    """f1 and f2 imported from arrays at every alignment come back as they were stored."""
+    from lbm_b200 import Lbm, Params
+    p = Params(nx=nx, ny=3, nz=4, nl=nl, iturb_pos=2, storage=storage)
+    L = Lbm(p)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nx + nl)
+    n = L.empty_f().numel()
+    m = [torch.ones(p.sshape, device="cuda") for _ in range(4)]
+    base = [1.0 / 27.0 + 1e-3 * torch.randn(n + 8, device="cuda", generator=g) for _ in range(2)]
+    got = []
+    for o1, o2 in ((0, 0), (1, 2), (2, 3), (3, 1)):
+        f = [torch.empty(n + 8, device="cuda")[o:o + n].view(p.fshape) for o in (o1, o2)]
+        for x, b in zip(f, base):
+            x.copy_(b[:n].view(p.fshape))
+        L.state_import(*f, *m)
+        out = [torch.full(p.fshape, 5.0, device="cuda") for _ in range(2)]
+        L.state_export(*out)
+        got.append(out)
+        # FP32 offsets keep a unit in the last place of f; FP16 ones 2^-11 of |f - w| < 0.3
+        tol = 6e-8 if storage == "f32" else 2e-4
+        assert all(float((a - b).abs().max()) <= tol for a, b in zip(out, f))
+    assert all(torch.equal(a, b) for o in got[1:] for a, b in zip(o, got[0]))
