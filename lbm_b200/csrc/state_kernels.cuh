@@ -84,6 +84,9 @@ struct alignas(16) StepArgs {
     int soff[27];             // l*dstride
     long long poffb[27];      // poff and soff in bytes, for the pair kernel: a 64-bit constant operand
     long long soffb[27];      // per address instead of a sign-extended, scaled 32-bit offset
+    // Where these two arrays lie in the arguments matters to the pair kernel, for a reason not found:
+    // at 456 or 472 bytes D3Q27 FP16 512x256x256 takes 682 us and FP32 128x64x64 26.6, at 240, 480 or
+    // 512 bytes 709 and 28.0.  Measure both after adding a member in front of them.
 };
 
 __device__ __forceinline__ void flag_bad_density(int* status, float rho, float ux, float uy, float uz) {
