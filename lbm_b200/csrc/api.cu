@@ -1637,7 +1637,7 @@ int lbm_launch_count(lbm_ctx* c, int64_t* n) {
 int lbm_profile(lbm_ctx* c, int32_t enable) {
     if (!c) return LBM_ERR_ARG;
     if (enable && c->ev.empty()) {
-        c->ev.resize(2 * 1024);
+        c->ev.resize(3 * 682);   // whole triples: prof_begin drains them when the last one is used
         for (auto& e : c->ev) LBM_TRY(cuda_check(c, cudaEventCreate(&e), "cudaEventCreate"));
     }
     LBM_TRY(prof_drain(c));
