@@ -83,22 +83,35 @@ __device__ __forceinline__ Moments2 moments_rows2(const f2 (&f)[Q]) {
     return m;
 }
 
-// EmitConst of collide_rows.cuh for two cells (nK9 = -K9)
+// FUSED, in the functions below: products that go into a sum are fused with it, as
+// the compiler does in the one-cell kernels.  Rows of an odd length (ODD) take it:
+// they ran in a one-cell kernel once, and round no more often than there (error of
+// a step against 64 bits, 201x96x96 FP32: D3Q19 9.86e-8 of the state and 9.80e-8 in the
+// one-cell kernel, 1.02e-7 without; D3Q27 9.70e-8, 9.62e-8 and 1.00e-7), at the same
+// speed but for FP16 boxes that are periodic all round (D3Q19 201x150x97 73 -> 77 us).
+
+// EmitConst of collide_rows.cuh for two cells (nK9 = -K9, now = -ow with FUSED)
 struct EmitConst2 {
     f2 C0, D0, R45, R45o, K45, K135, nK9;
     f2 ux, uy, uz, vx, vy, vz;
     f2 axx, ayy, azz, axy2, axz2, ayz2, syz;
-    f2 ow[4];
+    f2 ow[4], now[4];
 };
 
-template <int Q, typename S, int L>
+template <int Q, typename S, bool FUSED, int L>
 __device__ __forceinline__ void emit_pair2(f2 (&fp)[Q], const EmitConst2& k, f2 cu, f2 cac, f2 cau) {
     const f2 ws = bc2(lat_w<Q>(L) * store_scale<S>());
     const f2 cu2 = mul2(cu, cu);
     const f2 E = mul2(ws, fma2(k.K45, cac, fma2(k.R45, cu2, k.C0)));
-    const f2 O = mul2(k.ow[lat_speed2(L)], fma2(k.nK9, cau, mul2(cu, fma2(k.K135, cac, fma2(k.R45o, cu2, k.D0)))));
-    fp[L] = add2(E, O);
-    fp[lat_opposite(L)] = sub2(E, O);
+    const f2 Y = fma2(k.nK9, cau, mul2(cu, fma2(k.K135, cac, fma2(k.R45o, cu2, k.D0))));
+    if constexpr (FUSED) {
+        fp[L] = fma2(k.ow[lat_speed2(L)], Y, E);
+        fp[lat_opposite(L)] = fma2(k.now[lat_speed2(L)], Y, E);
+    } else {
+        const f2 O = mul2(k.ow[lat_speed2(L)], Y);
+        fp[L] = add2(E, O);
+        fp[lat_opposite(L)] = sub2(E, O);
+    }
 }
 
 // cy*y + cz*z for the rows emitted below (leading coefficient +1)
@@ -111,7 +124,7 @@ __device__ __forceinline__ f2 lin2(f2 y, f2 z) {
     else return sub2(y, z);
 }
 
-template <int Q, typename S, int CY, int CZ>
+template <int Q, typename S, bool FUSED, int CY, int CZ>
 __device__ __forceinline__ void emit_row2(f2 (&fp)[Q], const EmitConst2& k) {
     using R = Row<Q, CY, CZ>;
     const f2 uyz = lin2<CY, CZ>(k.uy, k.uz);
@@ -119,12 +132,12 @@ __device__ __forceinline__ void emit_row2(f2 (&fp)[Q], const EmitConst2& k) {
     f2 ayz;
     if constexpr (CY != 0 && CZ != 0) ayz = (CY * CZ > 0) ? add2(k.syz, k.ayz2) : sub2(k.syz, k.ayz2);
     else ayz = (CY != 0) ? k.ayy : k.azz;
-    emit_pair2<Q, S, R::l0>(fp, k, uyz, ayz, vyz);
+    emit_pair2<Q, S, FUSED, R::l0>(fp, k, uyz, ayz, vyz);
     if constexpr (R::hasx) {
         const f2 bx = lin2<CY, CZ>(k.axy2, k.axz2);
         const f2 t = add2(k.axx, ayz);
-        emit_pair2<Q, S, R::lp>(fp, k, add2(uyz, k.ux), add2(t, bx), add2(vyz, k.vx));
-        emit_pair2<Q, S, R::lm>(fp, k, sub2(uyz, k.ux), sub2(t, bx), sub2(vyz, k.vx));
+        emit_pair2<Q, S, FUSED, R::lp>(fp, k, add2(uyz, k.ux), add2(t, bx), add2(vyz, k.vx));
+        emit_pair2<Q, S, FUSED, R::lm>(fp, k, sub2(uyz, k.ux), sub2(t, bx), sub2(vyz, k.vx));
     }
 }
 
@@ -138,7 +151,9 @@ __device__ __forceinline__ float vreman_nut(float bb, float amag, const CollideP
 // units in the last FP32 place).  The FP16-offset state keeps 11 significant
 // bits, so these errors vanish in its rounding, while the correctly rounded
 // forms cost a dozen instructions and a branch each; the FP32 state keeps the
-// correctly rounded forms.
+// correctly rounded forms, and so do rows of an odd length in either storage (FP16
+// D3Q27 201x150x97: 98 us a step against 102 with the approximate ones, 109 and 104
+// in a box that is periodic all round).
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -149,18 +164,18 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-// 1/x of both cells: correctly rounded for FP32 storage, approximate for FP16
-template <typename S>
+// 1/x of both cells: approximate with APPROX, else correctly rounded
+template <bool APPROX>
 __device__ __forceinline__ f2 rcp2(f2 x) {
-    if constexpr (sizeof(S) == 2) return make_float2(rcp_approx(x.x), rcp_approx(x.y));
+    if constexpr (APPROX) return make_float2(rcp_approx(x.x), rcp_approx(x.y));
     else return make_float2(__frcp_rn(x.x), __frcp_rn(x.y));
 }
 // Vreman eddy viscosity of both cells from B_beta and |alpha|^2 (see vreman_nut)
-template <typename S>
+template <bool APPROX>
 __device__ __forceinline__ f2 vreman_nut2(f2 bb, f2 sq, const CollideParams& cp) {
     const float tiny = 1.17549435e-38f;
-    if constexpr (sizeof(S) == 2) {
-        const f2 t = mul2(bb, rcp2<S>(make_float2(fmaxf(sq.x, tiny), fmaxf(sq.y, tiny))));
+    if constexpr (APPROX) {
+        const f2 t = mul2(bb, rcp2<true>(make_float2(fmaxf(sq.x, tiny), fmaxf(sq.y, tiny))));
         return make_float2(t.x > cp.eps ? __fmul_rn(cp.cvre, sqrt_approx(t.x)) : 0.0f,
                            t.y > cp.eps ? __fmul_rn(cp.cvre, sqrt_approx(t.y)) : 0.0f);
     } else {
@@ -178,7 +193,7 @@ struct CollideState2 {
     f2 K;
 };
 
-template <typename S>
+template <bool APPROX, bool FUSED>
 __device__ __forceinline__ CollideState2 collide_pre2(const Moments2& m, f2 drho, f2 rho, f2 ux, f2 uy, f2 uz,
                                                       const CollideParams& cp, float abl) {
     CollideState2 c;
@@ -186,13 +201,24 @@ __device__ __forceinline__ CollideState2 collide_pre2(const Moments2& m, f2 drho
     const f2 third = bc2(1.0f / 3.0f);
     const f2 rux = mul2(rho, ux), ruy = mul2(rho, uy), ruz = mul2(rho, uz);
     c.rux = rux; c.ruy = ruy; c.ruz = ruz;
-    const f2 s3 = mul2(m.s0, third);
-    const f2 axx = sub2(sub2(m.pxx, s3), mul2(rux, ux));
-    const f2 ayy = sub2(sub2(m.pyy, s3), mul2(ruy, uy));
-    const f2 azz = sub2(sub2(m.pzz, s3), mul2(ruz, uz));
-    const f2 axy = sub2(m.pxy, mul2(rux, uy));
-    const f2 axz = sub2(m.pxz, mul2(rux, uz));
-    const f2 ayz = sub2(m.pyz, mul2(ruy, uz));
+    f2 axx, ayy, azz, axy, axz, ayz;
+    if constexpr (FUSED) {
+        const f2 nx = mul2(ux, bc2(-1.0f)), ny = mul2(uy, bc2(-1.0f)), nz = mul2(uz, bc2(-1.0f)), n3 = bc2(-1.0f / 3.0f);
+        axx = fma2(rux, nx, fma2(m.s0, n3, m.pxx));
+        ayy = fma2(ruy, ny, fma2(m.s0, n3, m.pyy));
+        azz = fma2(ruz, nz, fma2(m.s0, n3, m.pzz));
+        axy = fma2(rux, ny, m.pxy);
+        axz = fma2(rux, nz, m.pxz);
+        ayz = fma2(ruy, nz, m.pyz);
+    } else {
+        const f2 s3 = mul2(m.s0, third);
+        axx = sub2(sub2(m.pxx, s3), mul2(rux, ux));
+        ayy = sub2(sub2(m.pyy, s3), mul2(ruy, uy));
+        azz = sub2(sub2(m.pzz, s3), mul2(ruz, uz));
+        axy = sub2(m.pxy, mul2(rux, uy));
+        axz = sub2(m.pxz, mul2(rux, uz));
+        ayz = sub2(m.pyz, mul2(ruy, uz));
+    }
     c.axx = axx; c.ayy = ayy; c.azz = azz; c.axy = axy; c.axz = axz; c.ayz = ayz;
     c.tr = add2(add2(axx, ayy), azz);
     f2 tau = bc2(cp.tau0);
@@ -210,19 +236,19 @@ __device__ __forceinline__ CollideState2 collide_pre2(const Moments2& m, f2 drho
         f2 bb = sub2(mul2(b11, b22), mul2(b12, b12));
         bb = add2(bb, sub2(mul2(b11, b33), mul2(b13, b13)));
         bb = add2(bb, sub2(mul2(b22, b33), mul2(b23, b23)));
-        const f2 nut = vreman_nut2<S>(bb, sq, cp);
+        const f2 nut = vreman_nut2<APPROX>(bb, sq, cp);
         tau = fma2(bc2(3.0f), add2(bc2(cp.kinevisc + abl), nut), bc2(0.5f));
     }
-    c.K = sub2(bc2(1.0f), rcp2<S>(tau));
+    c.K = sub2(bc2(1.0f), rcp2<APPROX>(tau));
     return c;
 }
 
 // collide_rows() for two cells: fp receives the post-collision offsets times
 // store_scale<S>().  solid.x / solid.y flag the two cells.
-template <int Q, typename S>
+template <int Q, typename S, bool APPROX, bool FUSED>
 __device__ __forceinline__ void collide_rows2(f2 (&fp)[Q], const Moments2& m, f2 drho, f2 rho, f2 ux, f2 uy, f2 uz,
                                               const CollideParams& cp, float abl, bool solid0, bool solid1) {
-    const CollideState2 c = collide_pre2<S>(m, drho, rho, ux, uy, uz, cp, abl);
+    const CollideState2 c = collide_pre2<APPROX, FUSED>(m, drho, rho, ux, uy, uz, cp, abl);
     const f2 axx = c.axx, ayy = c.ayy, azz = c.azz, axy = c.axy, axz = c.axz, ayz = c.ayz, tr = c.tr, K = c.K;
     const bool cubic = (cp.ibgk == 3);
     const f2 usq = fma2(ux, ux, fma2(uy, uy, mul2(uz, uz)));
@@ -230,8 +256,15 @@ __device__ __forceinline__ void collide_rows2(f2 (&fp)[Q], const Moments2& m, f2
     k.R45 = mul2(bc2(4.5f), rho);
     k.R45o = cubic ? k.R45 : bc2(0.0f);
     const f2 ktr = mul2(K, tr);
-    k.C0 = sub2(sub2(drho, mul2(bc2(1.5f), mul2(rho, usq))), mul2(bc2(1.5f), ktr));
-    k.D0 = sub2(sub2(mul2(bc2(3.0f), rho), cubic ? mul2(k.R45, usq) : bc2(0.0f)), mul2(bc2(4.5f), ktr));
+    if constexpr (FUSED) {
+        k.C0 = fma2(bc2(-1.5f), ktr, fma2(bc2(-1.5f), mul2(rho, usq), drho));
+        k.D0 = mul2(bc2(3.0f), rho);
+        if (cubic) k.D0 = fma2(mul2(k.R45, bc2(-1.0f)), usq, k.D0);
+        k.D0 = fma2(bc2(-4.5f), ktr, k.D0);
+    } else {
+        k.C0 = sub2(sub2(drho, mul2(bc2(1.5f), mul2(rho, usq))), mul2(bc2(1.5f), ktr));
+        k.D0 = sub2(sub2(mul2(bc2(3.0f), rho), cubic ? mul2(k.R45, usq) : bc2(0.0f)), mul2(bc2(4.5f), ktr));
+    }
     k.K45 = mul2(bc2(4.5f), K);
     k.K135 = mul2(bc2(13.5f), K);
     k.nK9 = mul2(bc2(-9.0f), K);
@@ -250,13 +283,15 @@ __device__ __forceinline__ void collide_rows2(f2 (&fp)[Q], const Moments2& m, f2
         k.ow[1] = mul2(sg, bc2(lat_w<Q>(1)));
         k.ow[2] = mul2(sg, bc2(lat_w<Q>(7)));
         k.ow[3] = (Q == 27) ? mul2(sg, bc2(lat_w<27>(19))) : bc2(0.0f);
+        if constexpr (FUSED)
+            for (int q = 1; q < 4; ++q) k.now[q] = mul2(k.ow[q], bc2(-1.0f));
     }
     fp[0] = mul2(bc2(lat_w<Q>(0) * store_scale<S>()), k.C0);
-    emit_pair2<Q, S, Row<Q, 0, 0>::lp>(fp, k, ux, axx, k.vx);
-    emit_row2<Q, S, 0, 1>(fp, k);
-    emit_row2<Q, S, 1, 0>(fp, k);
-    emit_row2<Q, S, 1, 1>(fp, k);
-    emit_row2<Q, S, 1, -1>(fp, k);
+    emit_pair2<Q, S, FUSED, Row<Q, 0, 0>::lp>(fp, k, ux, axx, k.vx);
+    emit_row2<Q, S, FUSED, 0, 1>(fp, k);
+    emit_row2<Q, S, FUSED, 1, 0>(fp, k);
+    emit_row2<Q, S, FUSED, 1, 1>(fp, k);
+    emit_row2<Q, S, FUSED, 1, -1>(fp, k);
 }
 
 // Pull loads of the pair (i, i+1): direction L reads the pair at base + poff[L]
@@ -310,6 +345,7 @@ struct SepArraySink {
 // or a captured FP32 copy finished by a second kernel -- measured slower on B200.)
 template <int Q, typename S, bool FORCE = false, bool ODD = false>
 __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int i, int j, int k) {
+    constexpr bool APPROX = sizeof(S) == 2 && !ODD, FUSED = ODD;
     Moments2 m = moments_rows2<Q>(fp);
     if constexpr (sizeof(S) == 2) {
         const f2 is = bc2(1.0f / store_scale<S>());
@@ -319,7 +355,7 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
     }
     const f2 drho = m.s0;
     const f2 rho = add2(bc2(1.0f), m.s0);
-    const f2 inv = rcp2<S>(rho);
+    const f2 inv = rcp2<APPROX>(rho);
     const f2 ux = mul2(m.jx, inv), uy = mul2(m.jy, inv), uz = mul2(m.jz, inv);
     const f2 chk = add2(add2(rho, ux), add2(uy, uz));
     const bool tail = ODD && i == a.g.nx;
@@ -343,7 +379,7 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
     if constexpr (Q == 27 && sizeof(S) == 2) {
         // FP16-offset D3Q27: the separable transform of sep_emit.cuh, the turbulence
         // increment folded into its coefficients
-        const CollideState2 c = collide_pre2<S>(m, drho, rho, ux, uy, uz, a.cp, abl);
+        const CollideState2 c = collide_pre2<APPROX, FUSED>(m, drho, rho, ux, uy, uz, a.cp, abl);
         const bool cubic = a.cp.ibgk == 3;
         SepCoef t = sep_coefficients<S>(c, make_float2(solid0 ? -1.0f : 1.0f, solid1 ? -1.0f : 1.0f), cubic);
         if (a.uu != nullptr && (i == a.iturb || i + 1 == a.iturb)) {
@@ -357,7 +393,7 @@ __device__ __forceinline__ void pair_collide(f2 (&fp)[Q], const StepArgs& a, int
     } else
 #endif
     {
-    collide_rows2<Q, S>(fp, m, drho, rho, ux, uy, uz, a.cp, abl, solid0, solid1);
+    collide_rows2<Q, S, APPROX, FUSED>(fp, m, drho, rho, ux, uy, uz, a.cp, abl, solid0, solid1);
     if (a.uu != nullptr && (i == a.iturb || i + 1 == a.iturb)) {
         const int c = a.iturb - i;
         float t[Q];
