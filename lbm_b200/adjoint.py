@@ -157,8 +157,11 @@ class FusedProbeProblem:
     step 0) with a snapshot after step 0.  Each segment is replayed from its
     snapshot, each step writing its state buffer into an array of its own
     (``lbm_step_to``).  The last segment needs no replay: the forward's own steps
-    write their states into such arrays.  A step that a snapshot follows writes
-    its state straight into the snapshot."""
+    write their states into such arrays, at most ``checkpoint`` of them, which
+    stay until ``backward`` has used them (or the next ``forward``, or ``close``):
+    after it a problem holds its snapshots and the two state arrays that its
+    context is on.  A second ``backward`` replays the last segment like the others.
+    A step that a snapshot follows writes its state straight into the snapshot."""
 
     def __init__(self, params: Params, probes, nsteps: int, blanking=None, checkpoint: int = 10):
         if params.storage != "f32":
@@ -308,6 +311,7 @@ class FusedProbeProblem:
         g = torch.empty(self.p.fshape, device="cuda")        # the export writes every cell
         L.state_adjoint_export(g, A)
         main.synchronize()
+        self._last = None                    # another problem may take the arrays; but see _live
         del sets
         return g, uvel_h
 

@@ -1,6 +1,6 @@
 """The fused gradient over every way its steps fall into segments: a single one, full and
 short last ones, one step each; with and without overlap, twice in a row, and from a
-forward run that kept another run's arrays before."""
+forward run that kept another run's arrays before.  What a problem holds after it."""
 import numpy as np
 import pytest
 
@@ -51,3 +51,36 @@ def test_segments_give_the_percall_gradient(nsteps, K):
     assert float((a.forward(f1, f2, uvel, keep=False) - ru).abs().max()) < 1e-6
     a.close()
     ref.close()
+
+
+def small_problem(nsteps, K, nx=20):
+    from lbm_b200 import Lbm, Params
+    from lbm_b200.adjoint import FusedProbeProblem, initial_state
+    p = Params(nx=nx, ny=8, nz=8, nl=19, iturb_pos=2)
+    m = [torch.zeros(p.sshape, device="cuda") for _ in range(4)]
+    m[0][1:-1, 1:-1, 1:-1] = 1.0
+    uvel = torch.full((p.nz,), 0.05, device="cuda")
+    with Lbm(p) as L:
+        f1, f2 = initial_state(L, *m, uvel)
+        torch.cuda.synchronize()
+    cells = np.array([[3, 2, 2], [15, 5, 7], [10, 3, 4]])
+    return FusedProbeProblem(p, cells, nsteps, checkpoint=K), f1, f2, uvel
+
+
+@pytest.mark.parametrize("nsteps,K", [(6, 6), (12, 6), (15, 6), (18, 6)])
+@pytest.mark.parametrize("overlap", [True, False])
+def test_backward_gives_the_kept_states_back(nsteps, K, overlap):
+    """After a gradient a problem holds its checkpoints and two states, whatever the number of
+    segments; the arrays of the last segment and of the replays are free again."""
+    a, f1, f2, uvel = small_problem(nsteps, K)
+    uhat = torch.ones((3, 3), device="cuda")
+    base = torch.cuda.memory_allocated()
+    state = a.lbm.state_bytes()
+    for _ in range(2):
+        a.forward(f1, f2, uvel)
+        for _ in range(2):
+            a.backward(uhat, overlap=overlap)
+            bound = 2 * state + sum(t.numel() * 4 for c in a.ckpt.values() for t in (c if isinstance(c, tuple) else (c,)))
+            assert torch.cuda.memory_allocated() - base < bound + state // 2      # less than a third state
+    a.close()
+    assert torch.cuda.memory_allocated() - base < state // 2
