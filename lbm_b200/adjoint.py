@@ -246,27 +246,29 @@ class FusedProbeProblem:
         R = self._replayer() if overlap else L
         main = L.stream
         rep = R.stream
+        nsets = 2 if overlap else 1
+        kept, self._last = self._last, None
+        # The arrays of the replayed segments (segment q takes set q mod nsets), made before
+        # the replay stream waits for main: made later, they could be memory that a temporary of
+        # the adjoint steps has just given back, which main may not have read yet.  Set 0
+        # begins with the arrays the forward kept, whose segment is done by the time of a
+        # replay into it, but for those that the checkpoints or the context hold.
+        sets = [[] for _ in range(nsets)]
+        if kept is not None and len(segs) > nsets:
+            held = [self.ckpt[0][1]] + self._live
+            sets[0] = [t for t in kept if all(t is not h for h in held)]
+        for b in {q % nsets for q in range(0 if kept is None else 1, len(segs))}:
+            sets[b] += [L.state_scratch() for _ in range(min(self.K, self.nsteps) - len(sets[b]))]
+        released = [None] * nsets            # event: the adjoint is done with a set
         rep.wait_stream(main)                # the forward's snapshots and the seed are written on main
         R.set_inflow(self.uvel)
-        nsets = 2 if overlap else 1
-        sets = [None] * nsets                # arrays of a replayed segment, made when a replay first needs them
-        released = [None] * nsets            # event: the adjoint is done with a set
 
         def replay(q):
             """The states of segment q: P[n - s] after step n, and the input of step s."""
             s, b = segs[q], q % nsets
             e = min(s + self.K, self.nsteps)
-            if q == 0 and self._last is not None:
-                return (self.ckpt[0][0] if s == 0 else self.ckpt[s]), self._last, None
-            if sets[b] is None:
-                # set 0 begins with the arrays the forward kept, whose segment is done by now (a
-                # second call then replays that one too), but for the context's own two
-                sets[b] = []
-                if b == 0 and self._last is not None:
-                    held = [self.ckpt[0][1]] + self._live
-                    sets[b] = [t for t in self._last if all(t is not h for h in held)]
-                    self._last = None
-                sets[b] += [L.state_scratch() for _ in range(self.K - len(sets[b]))]
+            if q == 0 and kept is not None:
+                return (self.ckpt[0][0] if s == 0 else self.ckpt[s]), kept, None
             P = list(sets[b][:e - s])
             with torch.cuda.stream(rep):
                 if released[b] is not None:
@@ -311,8 +313,6 @@ class FusedProbeProblem:
         g = torch.empty(self.p.fshape, device="cuda")        # the export writes every cell
         L.state_adjoint_export(g, A)
         main.synchronize()
-        self._last = None                    # another problem may take the arrays; but see _live
-        del sets
         return g, uvel_h
 
     def close(self):

@@ -84,3 +84,24 @@ def test_backward_gives_the_kept_states_back(nsteps, K, overlap):
             assert torch.cuda.memory_allocated() - base < bound + state // 2      # less than a third state
     a.close()
     assert torch.cuda.memory_allocated() - base < state // 2
+
+
+@pytest.mark.parametrize("nsteps,K", [(6, 6), (9, 3), (14, 3)])
+@pytest.mark.parametrize("overlap", [True, False])
+def test_replay_arrays_are_made_before_the_adjoint_steps(nsteps, K, overlap, monkeypatch):
+    """The replay stream is ordered behind what was queued when the sweep began, so an array
+    made for it later could be memory that the adjoint stream has still to read."""
+    a, f1, f2, uvel = small_problem(nsteps, K)
+    uhat = torch.ones((3, 3), device="cuda")
+    calls = []
+    scratch, step = a.lbm.state_scratch, a.lbm.state_adjoint_step
+    monkeypatch.setattr(a.lbm, "state_scratch", lambda: (calls.append("array"), scratch())[1])
+    monkeypatch.setattr(a.lbm, "state_adjoint_step", lambda *x: (calls.append("step"), step(*x))[1])
+    for _ in range(2):
+        a.forward(f1, f2, uvel)
+        for _ in range(2):
+            calls.clear()
+            a.backward(uhat, overlap=overlap)
+            assert calls.count("step") == nsteps
+            assert "array" not in calls[calls.index("step"):]
+    a.close()
