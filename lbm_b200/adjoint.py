@@ -284,6 +284,8 @@ class FusedProbeProblem:
                     start = s
                 for n in range(start, e):
                     R.step_to(P[n - s])      # the step writes its state into the array
+                if R is L:
+                    self._live = P[-2:]
                 ready = torch.cuda.Event()
                 ready.record(rep)
             return first, P, ready

@@ -105,3 +105,18 @@ def test_replay_arrays_are_made_before_the_adjoint_steps(nsteps, K, overlap, mon
             assert calls.count("step") == nsteps
             assert "array" not in calls[calls.index("step"):]
     a.close()
+
+
+def test_the_context_keeps_its_state_after_a_serial_backward():
+    """Without overlap the forward's own context replays; the arrays it ends on stay with it."""
+    a, f1, f2, uvel = small_problem(13, 4)
+    a.forward(f1, f2, uvel)
+    a.backward(torch.ones((3, 3), device="cuda"), overlap=False)
+    M = [torch.empty(a.p.sshape, device="cuda") for _ in range(4)]
+    a.lbm.get_macro(*M)
+    fill = [a.lbm.state_scratch().fill_(float("nan")) for _ in range(12)]       # whatever was given back
+    N = [torch.empty(a.p.sshape, device="cuda") for _ in range(4)]
+    a.lbm.get_macro(*N)
+    assert all(torch.equal(x, y) for x, y in zip(M, N))
+    del fill
+    a.close()
