@@ -532,10 +532,10 @@ cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream
 bool pair_ok(const lbm_ctx* c) { return c->kernel == LBM_KERNEL_PAIR && c->p.ihrr == 1 && c->p.nx >= 4; }
 bool pair_even_ok(const lbm_ctx* c) { return pair_ok(c) && c->p.nx % 2 == 0; }
 
-template <int Q, typename S, bool WRAP, bool FORCE, bool FOLD, int T, bool ODD = false>
+template <int Q, typename S, bool WRAP, bool FORCE, bool FOLD, int T, bool ODD = false, bool PERI = !FOLD>
 cudaError_t pair_launch(lbm_ctx* c, const S* src, S* dst, const StepArgs& a) {
     const dim3 grd((unsigned)(((c->p.nx + 1) / 2 + T - 1) / T), c->p.ny, c->p.nz);
-    return launch_pdl(k_step_pair<Q, S, WRAP, FORCE, FOLD, T, ODD>, grd, dim3(T), c->stream, src, dst, a);
+    return launch_pdl(k_step_pair<Q, S, WRAP, FORCE, FOLD, T, ODD, PERI>, grd, dim3(T), c->stream, src, dst, a);
 }
 
 // the steady step from buffer cur into nxt, two cells per thread
@@ -553,6 +553,9 @@ int pair_family_step(lbm_ctx* c, int nxt, const StepArgs& a) {
                         : pair_launch<Q, S, WRAP, false, FOLD, 128, true>(c, src, dst, a);
         else
             r = cudaErrorInvalidValue;
+    } else if (c->force && !FOLD && !a.peri) {
+        r = t == 256 ? pair_launch<Q, S, WRAP, true, FOLD, W, false, false>(c, src, dst, a)
+                     : pair_launch<Q, S, WRAP, true, FOLD, 128, false, false>(c, src, dst, a);
     } else if (c->force) {
         r = t == 256 ? pair_launch<Q, S, WRAP, true, FOLD, W>(c, src, dst, a)
                      : pair_launch<Q, S, WRAP, true, FOLD, 128>(c, src, dst, a);

@@ -457,12 +457,12 @@ __device__ __forceinline__ void pair_edge(const f2 (&fp)[Q], const StepArgs& a, 
 
 // Everything after the loads of one pair: pair_collide, the stores and the edge
 // copy of the folded boundaries (FOLD).
-template <int Q, typename S, bool FOLD, bool FORCE = false, bool ODD = false>
+template <int Q, typename S, bool FOLD, bool FORCE = false, bool ODD = false, bool PERI = !FOLD>
 __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, const StepArgs& a, long long o, int i,
                                             int j, int k) {
     pair_collide<Q, S, FORCE, ODD>(fp, a, i, j, k);
     S* q = dst + o;
-    if (!FOLD && a.peri && (i == 1 || i + 2 > a.g.nx)) {
+    if (PERI && a.peri && (i == 1 || i + 2 > a.g.nx)) {
         // periodic i: the ghosts nx+1 and 0 of this row from the cells 1 and nx
 #pragma unroll
         for (int l = 0; l < Q; ++l) {
@@ -521,8 +521,11 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
 // One pair (i, i+1), i odd, of row (j, k): pull, collide, store.  WRAP: periodic
 // j read through rows ny and 1; FOLD: the folded boundaries follow (edge copy).
 // A j-slab tile in the folded configuration pulls its stored halo planes
-// (WRAP false) and keeps the folded boundaries (FOLD true).
-template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, bool ODD = false>
+// (WRAP false) and keeps the folded boundaries (FOLD true).  PERI: compiled for
+// periodic boxes too (StepArgs::peri).  The forced kernels come with and without
+// it: the i ghosts' stores cost D3Q27 FP32 72 bytes of spills more, 173 us against
+// 164 for 256x128x128 in a box that has closed faces.
+template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, bool ODD = false, bool PERI = !FOLD>
 __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restrict__ dst, const StepArgs& a, int i, int j,
                                           int k) {
     const long long o = a.g.off(i, j, k);
@@ -534,7 +537,7 @@ __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restri
         const S* pym = (WRAP && j == a.g.ny) ? p0 - wrapd : p0;
         PairLoad<Q, S, 0>::run(fp, p0, pyp, pym, a);
     }
-    pair_update<Q, S, FOLD, FORCE, ODD>(fp, dst, a, o, i, j, k);
+    pair_update<Q, S, FOLD, FORCE, ODD, PERI>(fp, dst, a, o, i, j, k);
 }
 
 #ifndef LBM_PAIR_MIN_BLOCKS
@@ -571,13 +574,13 @@ inline int pair_width(int hp) {
 }
 // Grid: x covers the row's pairs in blocks of T threads, y = j, z = k.  Needs
 // ihrr = 1 (and an even nx without ODD); offsets are 64-bit, so any state size.
-template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, int T = 128, bool ODD = false>
+template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, int T = 128, bool ODD = false, bool PERI = !FOLD>
 __global__ void __launch_bounds__(T, pair_min_blocks<Q, S, T>()) k_step_pair(const S* __restrict__ src, S* __restrict__ dst,
                                                                              StepArgs a) {
     pdl_enter();
     const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + 1;
     if (i > a.g.nx) return;
-    pair_cell<Q, S, WRAP, FORCE, FOLD, ODD>(src, dst, a, i, blockIdx.y + 1, blockIdx.z + 1);
+    pair_cell<Q, S, WRAP, FORCE, FOLD, ODD, PERI>(src, dst, a, i, blockIdx.y + 1, blockIdx.z + 1);
 }
 
 // macrovars of the reference's f1 without materialising it: interior cells from

@@ -36,13 +36,13 @@ def test_forcings_apply_per_call(nl):
     assert e64 <= 1.5 * floor + 1e-9 and e32 <= 2.5 * floor + 1e-9, (e64, e32, floor)
 
 
-def run_forced(wl, steps, storage, F, kernel=None):
+def run_forced(wl, steps, storage, F, kernel=None, slice_on=True):
     from lbm_b200 import Solver
     blank = W.blanking(wl)
     rho, u, v, w = (cuda(a) for a in W.initial_macro(wl))
     uvel = cuda(W.inflow_profile(wl))
     turb = W.turbulence_fields(wl.ny, wl.nz, wl.nrturb, 3)
-    tb = (cuda(turb[0]), cuda(turb[1]), cuda(turb[2]), wl.nrturb, wl.ampl)
+    tb = (cuda(turb[0]), cuda(turb[1]), cuda(turb[2]), wl.nrturb, wl.ampl) if slice_on else None
     s = Solver(params_of(wl, iturb_pos=5, storage=storage), rho, u, v, w, uvel, blanking=cuda(blank), turbulence=tb)
     if kernel:
         s.lbm.set_kernel(kernel)
@@ -56,11 +56,11 @@ def run_forced(wl, steps, storage, F, kernel=None):
     return out
 
 
-def oracle_forced(wl, steps, dtype, F):
+def oracle_forced(wl, steps, dtype, F, slice_on=True):
     blank = W.blanking(wl)
     turb = W.turbulence_fields(wl.ny, wl.nz, wl.nrturb, 3)
     cfg = O.Config(wl.nx, wl.ny, wl.nz, wl.nl, ibnd=wl.ibnd, jbnd=wl.jbnd, kbnd=wl.kbnd, iturb_pos=5, lsolids=True,
-                   lturb=True, nrturb=wl.nrturb, kinevisc=wl.kinevisc, ampl=wl.ampl)
+                   lturb=slice_on, nrturb=wl.nrturb, kinevisc=wl.kinevisc, ampl=wl.ampl)
     o = O.Oracle(cfg, dtype)
     rho, u, v, w = (a.astype(dtype) for a in W.initial_macro(wl))
     uvel = W.inflow_profile(wl, dtype)
@@ -82,6 +82,23 @@ def test_fused_forcing_matches_oracle(nl):
     # the forcing does something: without it the run differs well beyond the floor
     unforced = run_forced(wl, wl.steps, "f32", np.zeros_like(F))
     assert rel_l2(unforced[3], ref64[3]) > 100 * rel_l2(gpu[3], ref64[3])
+
+
+@pytest.mark.parametrize("codes", [(0, 0, 0), (11, 0, 22), (12, 0, 0), (1, 11, 22)])
+@pytest.mark.parametrize("nl,storage,nx", [(19, "f32", 16), (27, "f32", 34), (27, "f16", 34), (27, "f16", 512)])
+def test_fused_forcing_outside_the_folded_configuration(codes, nl, storage, nx):
+    """Periodic boxes, where the forced kernel writes the i ghosts, and boxes with closed faces,
+    where an instance without those stores runs; FP16 D3Q27 in both widths of block."""
+    ib, jb, kb = codes
+    wl = SMALL.with_(nl=nl, nx=nx, ny=6, nz=5, ibnd=ib, jbnd=jb, kbnd=kb)
+    F = (2e-5 * np.random.default_rng(9).standard_normal((wl.nz + 2, wl.ny + 2, wl.nx + 2, 3))).astype(np.float32)
+    gpu = run_forced(wl, 10, storage, F, slice_on=False)
+    ref32, ref64 = (oracle_forced(wl, 10, dt, F, slice_on=False) for dt in (np.float32, np.float64))
+    if storage == "f32":
+        compare_to_floor(gpu, ref32, ref64, "forced, codes %s" % (codes,))
+    else:
+        s = (slice(1, -1),) * 3
+        assert rel_l2(np.stack(gpu[3:])[(slice(None),) + s], np.stack(ref64[3:])[(slice(None),) + s]) < 1e-3
 
 
 def test_fused_forcing_fp16_storage():
