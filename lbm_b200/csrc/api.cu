@@ -553,9 +553,8 @@ int pair_family_step(lbm_ctx* c, int nxt, const StepArgs& a) {
                         : pair_launch<Q, S, WRAP, false, FOLD, 128, true>(c, src, dst, a);
         else
             r = cudaErrorInvalidValue;
-    } else if (c->force && !FOLD && !a.peri) {
-        r = t == 256 ? pair_launch<Q, S, WRAP, true, FOLD, W, false, false>(c, src, dst, a)
-                     : pair_launch<Q, S, WRAP, true, FOLD, 128, false, false>(c, src, dst, a);
+    } else if (c->force && sizeof(S) == 4 && !a.peri) {
+        r = pair_launch<Q, S, WRAP, true, FOLD, 128, false, sizeof(S) == 2 && !FOLD>(c, src, dst, a);
     } else if (c->force) {
         r = t == 256 ? pair_launch<Q, S, WRAP, true, FOLD, W>(c, src, dst, a)
                      : pair_launch<Q, S, WRAP, true, FOLD, 128>(c, src, dst, a);

@@ -522,9 +522,11 @@ __device__ __forceinline__ void pair_update(f2 (&fp)[Q], S* __restrict__ dst, co
 // j read through rows ny and 1; FOLD: the folded boundaries follow (edge copy).
 // A j-slab tile in the folded configuration pulls its stored halo planes
 // (WRAP false) and keeps the folded boundaries (FOLD true).  PERI: compiled for
-// periodic boxes too (StepArgs::peri).  The forced kernels come with and without
-// it: the i ghosts' stores cost D3Q27 FP32 72 bytes of spills more, 173 us against
-// 164 for 256x128x128 in a box that has closed faces.
+// periodic boxes too (StepArgs::peri).  The forced FP32 kernels come with and without
+// it: the i ghosts' stores cost D3Q27 72 bytes of spills more, 173 us against 164 for
+// 256x128x128 in a box that has closed faces (D3Q19 128.4 and 127.0).  The forced FP16
+// kernels come with it only: D3Q27 spills less then (360 bytes, 392 without), 167 us
+// against 182.
 template <int Q, typename S, bool WRAP, bool FORCE = false, bool FOLD = WRAP, bool ODD = false, bool PERI = !FOLD>
 __device__ __forceinline__ void pair_cell(const S* __restrict__ src, S* __restrict__ dst, const StepArgs& a, int i, int j,
                                           int k) {
