@@ -398,10 +398,9 @@ int bc_ref(lbm_ctx* c, R* f1, R* f2, const R* uvel) {
         if (codes[a] == 0 && !(wrap && a == 1)) periodic(a);
     for (int a = 0; a < 3; ++a) {
         if (!c->face_on[a]) continue;
-        const int np = std::max(c->face[a][0].n, c->face[a][1].n);
-        const long long na = (long long)(a == 0 ? ny : nx) * np;   // threads over the first tangential extent
+        const long long na = (long long)(a == 0 ? ny : nx) * ClosedPairs<Q>::N;   // threads over the first tangential extent
         const int nb = (a == 2) ? ny : nz;
-        k_ref_closed<Q, R><<<dim3((unsigned)((na + 127) / 128), nb, 2), 128, 0, s>>>(f1, f2, g, a, c->face[a][0],
+        k_ref_closed<Q, R><<<dim3((unsigned)((na + 127) / 128), nb), 128, 0, s>>>(f1, f2, g, a, c->face[a][0],
                                                                                     c->face[a][1], wrap ? 1 : 0);
         c->launches++;
     }
