@@ -9,10 +9,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nsteps,K", [(1, 1), (2, 1), (5, 1), (3, 10), (4, 4), (8, 4), (9, 4), (11, 4), (13, 3)])
-def test_segments_give_the_percall_gradient(nsteps, K):
+def test_segments_give_the_percall_gradient(nsteps, K, nx=20):
     from lbm_b200 import Lbm, Params
     from lbm_b200.adjoint import FusedProbeProblem, ProbeProblem, initial_state
-    p = Params(nx=20, ny=6, nz=8, nl=19, iturb_pos=2)
+    p = Params(nx=nx, ny=6, nz=8, nl=19, iturb_pos=2)
     g = torch.Generator(device="cuda")
     g.manual_seed(nsteps * 16 + K)
     m = [torch.zeros(p.sshape, device="cuda") for _ in range(4)]
@@ -51,6 +51,11 @@ def test_segments_give_the_percall_gradient(nsteps, K):
     assert float((a.forward(f1, f2, uvel, keep=False) - ru).abs().max()) < 1e-6
     a.close()
     ref.close()
+
+
+@pytest.mark.parametrize("nsteps,K,nx", [(9, 4, 21), (13, 3, 23)])
+def test_segments_of_odd_rows(nsteps, K, nx):
+    test_segments_give_the_percall_gradient(nsteps, K, nx)
 
 
 def small_problem(nsteps, K, nx=20):

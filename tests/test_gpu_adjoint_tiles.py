@@ -1,7 +1,6 @@
 """The adjoint kernels at the edges of their tiles: the drift transpose against its
-definition, the boundary transpose against its forward (a linear map), the collision
-adjoint of a row against the same cells elsewhere in a row, and the reverse step in
-pairs against one cell at a time."""
+definition, the boundary transpose against its forward (a linear map), and the collision
+adjoint of a row against the same cells elsewhere in a row."""
 import pytest
 
 from tests.test_gpu_percall_tiles import C, SHAPES, at_offset, equilibrium_like, lbm_of

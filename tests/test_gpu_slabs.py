@@ -90,15 +90,22 @@ def gpu_tiles(wl, ntiles, steps, storage="f32", kernel=None):
 
 
 @pytest.mark.parametrize("nl,ntiles,codes", [(19, 2, (1, 0, 12)), (27, 3, (1, 0, 12)), (19, 2, (11, 0, 22)),
-                                             (27, 2, (1, 11, 22))])
-def test_tiles_match_tiled_oracle(nl, ntiles, codes):
+                                             (27, 2, (1, 11, 22)), (19, 3, (0, 0, 0)), (27, 2, (0, 0, 0))])
+def test_tiles_match_tiled_oracle(nl, ntiles, codes, nx=16):
     ib, jb, kb = codes
-    wl = W.Workload("slabs", 16, 12, 8, nl, steps=10, ibnd=ib, jbnd=jb, kbnd=kb, noise=3e-3, sphere=(6, 5, 4, 2))
+    wl = W.Workload("slabs", nx, 12, 8, nl, steps=10, ibnd=ib, jbnd=jb, kbnd=kb, noise=3e-3, sphere=(6, 5, 4, 2))
     gpu = gpu_tiles(wl, ntiles, wl.steps)
     ref32 = oracle_tiles(wl, ntiles, np.float32, wl.steps)
     ref64 = oracle_tiles(wl, ntiles, np.float64, wl.steps)
     for r in range(ntiles):
         compare_to_floor(gpu[r], ref32[r], ref64[r], "tile %d of %d, codes %s" % (r, ntiles, codes))
+
+
+@pytest.mark.parametrize("nl,ntiles,codes,nx", [(27, 2, (0, 0, 0), 17), (19, 2, (11, 0, 22), 17), (27, 3, (12, 0, 0), 15)])
+def test_tiles_of_odd_rows(nl, ntiles, codes, nx):
+    """The i ghosts from the step kernel's row ends, the other ghosts and the exchanged planes
+    meet at a row whose last pair holds one cell."""
+    test_tiles_match_tiled_oracle(nl, ntiles, codes, nx)
 
 
 @pytest.mark.parametrize("nl,storage", [(19, "f32"), (27, "f32"), (27, "f16")])
