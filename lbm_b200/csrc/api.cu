@@ -1004,6 +1004,14 @@ int lbm_create(lbm_ctx** out, const lbm_params* p) {
     return LBM_OK;
 }
 
+}  // extern "C"
+
+namespace {
+void turb_release(lbm_ctx* c);   // turbulence_host.cuh
+}
+
+extern "C" {
+
 int lbm_destroy(lbm_ctx* c) {
     if (!c) return LBM_ERR_ARG;
     cudaStreamSynchronize(c->stream);
@@ -1017,9 +1025,7 @@ int lbm_destroy(lbm_ctx* c) {
     for (int b = 0; b < 2; ++b) cudaFree(c->d_xg[b]);
     cudaFree(c->d_abl);
     cudaFree(c->d_adj_terms);
-    if (c->turb_planes > 0) cufftDestroy(c->turb_plan);
-    cudaFree(c->d_turb_buf);
-    cudaFree(c->d_turb_part);
+    turb_release(c);
     cudaFree(c->d_it);
     cudaFree(c->d_status);
     cudaFree(c->d_partial);

@@ -1,6 +1,8 @@
 // boundary.cuh -- ghost-cell kernels of boundarycond (m_boundarycond.F90:14-468),
-// written once against a layout accessor so that the per-call entry point
-// (reference layout) and the fused state (structure of arrays) share them.
+// written against a layout accessor.  The fused state (structure of arrays) runs
+// all of them where its boundaries are not folded; the per-call entry point
+// (reference layout) shares the edges and corners and has periodic, closed-face and
+// inflow kernels of its own (ref_kernels.cuh), as its cells keep their values together.
 //
 // Every kernel here reads and writes ghost cells only from the interior or
 // from the previous buffer, so threads never race: a closed-face thread writes
@@ -16,7 +18,6 @@ namespace lbm {
 // in the arithmetic type R (FP32, or FP64 for the DP build's entry points).
 template <typename R>
 struct AosAccT {
-    using real = R;
     R* f;
     RefGrid g;
     __device__ __forceinline__ R* p(int l, int i, int j, int k) const { return f + g.cell(i, j, k) * g.nl + l; }
@@ -33,7 +34,6 @@ using AosAcc = AosAccT<float>;
 // Accessor for the fused state: offsets f - w_l in storage type S.
 template <typename S>
 struct SoaAcc {
-    using real = float;
     S* f;
     SoaGrid g;
     __device__ __forceinline__ S* p(int l, int i, int j, int k) const { return f + (long long)l * g.dstride + g.off(i, j, k); }
@@ -155,28 +155,24 @@ __global__ void k_corners(Acc f1, Acc f2, CornerSet cs) {
 // fghost(l) = f(l,1,j,k) - 2 w_l rho0 (cx u cos + cy u sin) / cs2; directions with
 // cx > 0 take fghost of their opposite.  In offset storage w_l cancels, and
 // opposite directions share w_l, so the same update holds for f - w_l.
-// Acc::real is the arithmetic type (FP32 for the fused state and the default
-// entry point, FP64 for the DP one).
 template <int Q, typename Acc>
-__global__ void k_inflow(Acc f, const typename Acc::real* __restrict__ uvel, typename Acc::real rho0,
-                         typename Acc::real cosd, typename Acc::real sind) {
-    using R = typename Acc::real;
+__global__ void k_inflow(Acc f, const float* __restrict__ uvel, float rho0, float cosd, float sind) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int k = blockIdx.y + 1;
     const int nx = f.g.nx;
     if (j > f.g.ny) return;
-    const R uu = uvel[k - 1];
-    const R cs2 = R(1) / R(3);
-    R fg[Q];
+    const float uu = uvel[k - 1];
+    const float cs2 = 1.0f / 3.0f;
+    float fg[Q];
 #pragma unroll
     for (int l = 0; l < Q; ++l) {
-        const R wl = lat_w<Q, R>(l);
-        const R cxl = (R)lat_cx(l), cyl = (R)lat_cy(l);
-        fg[l] = f.ld(l, 1, j, k) - R(2) * wl * rho0 * (cxl * uu * cosd + cyl * uu * sind) / cs2;
+        const float wl = lat_w<Q>(l);
+        const float cxl = (float)lat_cx(l), cyl = (float)lat_cy(l);
+        fg[l] = f.ld(l, 1, j, k) - 2.0f * wl * rho0 * (cxl * uu * cosd + cyl * uu * sind) / cs2;
     }
 #pragma unroll
     for (int l = 0; l < Q; ++l) {
-        const R v = (lat_cx(l) <= 0) ? fg[l] : fg[lat_opposite(l)];
+        const float v = (lat_cx(l) <= 0) ? fg[l] : fg[lat_opposite(l)];
         f.st(l, 0, j, k, v);
     }
 #pragma unroll

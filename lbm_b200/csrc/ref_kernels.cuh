@@ -1,11 +1,12 @@
 // ref_kernels.cuh -- per-call kernels on the reference layout
 // f(nl,0:nx+1,0:ny+1,0:nz+1) (l fastest), one per reference subroutine.
 //
-// Cell-wise kernels stage a row chunk of 128 cells (128*nl contiguous values)
-// through shared memory, so the global reads and writes are coalesced even
-// though each cell's nl populations are contiguous; the per-cell math reads
-// the staged values with an odd stride (nl = 19 or 27), free of bank
-// conflicts for FP32.
+// Cell-wise kernels stage runs of cells (nl contiguous values each) through shared
+// memory, so the global reads and writes are coalesced even though each cell's nl
+// populations are contiguous; the per-cell math reads the staged values with an odd
+// stride (nl = 19 or 27), free of bank conflicts for FP32.  postcoll and macrovars walk
+// tiles of 64 or 128 cells that pass over row ends, the next one under way
+// (ref_tiles.cuh); the others take a chunk of 128 cells of a row.
 //
 // Every kernel takes the arithmetic type R as a template argument: float for
 // the reference's default build, double for its DP build (the _f64 entry
@@ -123,9 +124,15 @@ __global__ void __launch_bounds__(128) k_ref_fequil3(R* feq, const R* rho, const
 // `scalars` values per cell each; as many blocks as fit an SM, up to a cap on
 // their registers.
 // T: postcoll reads, computes and writes between three barriers, so more, smaller blocks
-// serve it where a block of 128 fills much of an SM: D3Q27 FP32 256x128x128 195 us in
-// tiles of 64 cells and 207 in tiles of 128, D3Q19 FP64 192x96x96 106 and 117; the
-// smaller D3Q19 FP32 tiles lose, 27.4 and 25.7 for 128x64x64.
+// serve it.  us in tiles of 64 and of 128 cells:
+//              128x64x64     192x96x96      256x128x128    512x128x128
+//   D3Q27 FP32 32.9  33.9    90.9  99.8     196.0 207.5    365.0 375.1
+//   D3Q27 FP64 52.8  60.2    155.4 180.5    334.9 371.5    642.5 681.6
+//   D3Q19 FP64 39.4  42.0    107.9 116.6    241.8 253.9    477.5 472.4
+//   D3Q19 FP32 29.1  27.4    70.9  74.2     165.8 173.8    300.3 307.8
+// D3Q19 FP32 was set to 128 on the first column alone, the one in which 64 loses; larger
+// grids would gain 2 to 5% from 64.  macrovars is within 2% (3% for D3Q27 FP32
+// 512x128x128) either way.
 template <int Q, typename R>
 struct PostcollTile {
     static constexpr int T = (sizeof(R) == 4 && Q == 19) ? 128 : 64;

@@ -25,6 +25,8 @@
 //     directions a pull reads (cx > 0 at i = 0, cx < 0 at nx+1).
 #pragma once
 
+#include <cstddef>
+
 #include "collide_rows.cuh"
 #include "ref_tiles.cuh"
 
@@ -84,10 +86,12 @@ struct alignas(16) StepArgs {
     int soff[27];             // l*dstride
     long long poffb[27];      // poff and soff in bytes, for the pair kernel: a 64-bit constant operand
     long long soffb[27];      // per address instead of a sign-extended, scaled 32-bit offset
-    // Where these two arrays lie in the arguments matters to the pair kernel, for a reason not found:
-    // at 456 or 472 bytes D3Q27 FP16 512x256x256 takes 682 us and FP32 128x64x64 26.6, at 240, 480 or
-    // 512 bytes 709 and 28.0.  Measure both after adding a member in front of them.
 };
+// The pair kernel is faster with the two byte tables 8 bytes past a multiple of 16 in the arguments
+// (at 456 and 472 bytes) than on one (at 240, 480 and 512, and with 8 bytes put in front of them):
+// D3Q27 FP16 512x256x256 681 and 707 us, FP32 1167 and 1178, FP32 128x64x64 26.6 and 28.1, with the
+// same registers and spills.  Why is not known; a member in front of them keeps them there.
+static_assert(offsetof(StepArgs, poffb) % 16 == 8, "the byte tables' place in the arguments (see above)");
 
 __device__ __forceinline__ void flag_bad_density(int* status, float rho, float ux, float uy, float uz) {
     const float chk = rho + ux + uy + uz;
